@@ -486,6 +486,7 @@ class OptImpl {
     uint64_t key = 0;
     bool verbose = false;
     std::function<void(int, cudaStream_t)> body, tail_body;
+    std::function<void(cudaStream_t)> post;  // after the iterations, on the stream they ran on
   };
 
   Plan plan(bool verbose, cudaStream_t st) {
@@ -500,6 +501,7 @@ class OptImpl {
     Plan p = plan(verbose, st);
     run_iterations(graph_, p.key, p.n, profiling_ ? p.n + 2 : kGraphIters, p.body, st, capture_stream());
     for (int i = 0; i < p.tail; ++i) p.tail_body((p.n + i) & 1, st);
+    if (p.post) p.post(st);
     finish(p);
   }
   const OpImpl* op_ptr() const { return op_.get(); }
@@ -643,6 +645,8 @@ class OptImpl {
     const int s = pingpong(f) ? set : 0;
     return static_cast<char*>(img_.p) + ((size_t)s * F_COUNT + f) * plane_bytes();
   }
+  // Plane f of half `set` of the slab, whatever the field's own rule.
+  void* raw_field(int f, int set) const { return static_cast<char*>(img_.p) + ((size_t)set * F_COUNT + f) * plane_bytes(); }
   ImgPtrs ptrs(int set) const {
     ImgPtrs p;
     p.u = field(F_U, set);
@@ -810,14 +814,18 @@ class OptImpl {
       r_reset_ = true;
       ++version_;
     }
+    const bool r_zero = r_reset_;
     if (r_reset_) {
       PDT_CUDA_CHECK(cudaMemsetAsync(r_.p, 0, r_.bytes, st));
       r_reset_ = false;
     }
+    // A line mask: an iteration is two launches (pdt_gram.h). Its set-up and the k-space dual at its end are
+    // two adjoints and one forward, which fewer than kGramMinIters iterations do not pay back.
+    const GramRows* gram = params_.max_iter + 1 >= kGramMinIters ? hk->line_gram() : nullptr;
     const int G = hk->groups();
     const long long gstride = hk->group_stride();
     const size_t khr_bytes = (size_t)G * gstride * sizeof(float2);
-    if (khr_.bytes != khr_bytes) {
+    if (!gram && khr_.bytes != khr_bytes) {
       khr_.ensure(khr_bytes);
       ++version_;
     }
@@ -830,19 +838,28 @@ class OptImpl {
     // alpha table for every iteration (tgvmrioptimizer.cu:144-155 in real_type)
     const unsigned K = params_.max_iter;
     const int n = (int)K + 1;
-    std::vector<float> tab(2 * (size_t)n);
+    const int ld = gram ? 4 : 2;  // with line_gram(): {alpha0, alpha1, c, d}, c and d as in pdt_gram.h
+    std::vector<float> tab(ld * (size_t)n);
+    double gc = 0, gd = 1;
+    const float gk = sigma / (1.0f + sigma * lambda);
     for (unsigned k = 0; k <= K; ++k) {
       float a0 = (float)params_.alpha0, a1 = (float)params_.alpha1;
       if (kind_ == PDT_OPT_TGV_MRI) alpha_at(k, a0, a1);
-      tab[2 * k] = a0;
-      tab[2 * k + 1] = a1;
+      tab[ld * k] = a0;
+      tab[ld * k + 1] = a1;
+      if (gram) {
+        gc += (double)gk * (1.0 - (double)lambda * gc);
+        gd -= (double)gk * (double)lambda * gd;
+        tab[ld * k + 2] = (float)gc;
+        tab[ld * k + 3] = (float)gd;
+      }
     }
     if (verbose) {
       print_params();
       for (unsigned k = 0; k <= K; ++k)
         if (params_.check && !(k % params_.check)) {
           if (kind_ == PDT_OPT_TGV_MRI)
-            std::cout << "iter=" << k << " alpha0=" << tab[2 * k] << " alpha1=" << tab[2 * k + 1] << std::endl;
+            std::cout << "iter=" << k << " alpha0=" << tab[ld * k] << " alpha1=" << tab[ld * k + 1] << std::endl;
           else
             std::cout << "iter=" << k << " lambda=" << lambda << std::endl;
         }
@@ -861,6 +878,7 @@ class OptImpl {
       alpha_host_ = tab;
     }
     PDT_CUDA_CHECK(cudaMemsetAsync(iter, 0, sizeof(int), st));  // the primal kernel advances it
+    if (gram) PDT_CUDA_CHECK(cudaMemsetAsync(iter + 4, 0, 2 * sizeof(int), st));  // or the one-launch iteration these
     const bool is_tgv = kind_ != PDT_OPT_TV_OP;
     const int p0 = parity_;
     const float* atab = reinterpret_cast<const float*>(alpha_.as<char>() + kAlphaHeader);
@@ -869,6 +887,10 @@ class OptImpl {
     pl.n = n;
     pl.p0 = p0;
     pl.verbose = verbose;
+    if (gram) {
+      plan_gram(pl, *gram, hk, r_zero, tau, sigma, lambda, gk, (float)gc, (float)gd, st);
+      return pl;
+    }
     ensure_aux();
     cudaStream_t aux = aux_;
     cudaEvent_t ev_fork = ev_fork_, ev_join = ev_join_;
@@ -904,6 +926,83 @@ class OptImpl {
                         (uintptr_t)is_tgv, (uintptr_t)fused, fbits(lambda), fbits(tau), fbits(sigma),
                         (uintptr_t)version_});
     return pl;
+  }
+
+  // The iterations with a line mask's row operator (pdt_gram.h): b = K^H f and z0 = K^H r_0, the first dual
+  // update and U; two launches an iteration; then the k-space dual from U. u, v, U alternate between two copies
+  // with the iteration (the free halves of the slab), p and q with the state's parity. An error of b acts like
+  // one of the data in every iteration, so its rows are transformed in FP32 (with the tensor-core rows u was
+  // 1.5e-6 off after 1001 iterations instead of 5e-7).
+  void plan_gram(Plan& pl, const GramRows& rows, SolverHooks* hk, bool r_zero, float tau, float sigma, float lambda,
+                 float k, float c, float d, cudaStream_t st) {
+    const size_t N = (size_t)W_ * H_, plane = plane_bytes();
+    const size_t bytes = (6 + (size_t)rows.groups) * plane;
+    if (gram_.bytes != bytes) {
+      gram_.ensure(bytes);
+      ++version_;
+    }
+    float2* U = gram_.as<float2>();  // two copies of {U, compensation}, b, z0, partial sums
+    float2* b = U + 4 * N;
+    float2* z0 = b + N;
+    float2* part = z0 + N;
+    hk->adjoint_compact(fc_.as<float2>(), b, st, true);
+    if (!r_zero) hk->adjoint_compact(r_.as<float2>(), z0, st, true);
+    const int p0 = parity_, n = pl.n;
+    const bool is_tgv = kind_ != PDT_OPT_TV_OP;
+    int* header = alpha_.as<int>();
+    const float4* table = reinterpret_cast<const float4*>(alpha_.as<char>() + kAlphaHeader);
+    {
+      // the first dual update reads {alpha0, alpha1} of row 0 whatever the row length
+      launch_mri_dual(is_tgv, W_, H_, ptrs(p0), ptrs(p0 ^ 1), sigma, reinterpret_cast<const float*>(table), header, st);
+      launch_gram_start(W_, H_, static_cast<const float2*>(field(F_UB, p0)), k, U, st);
+    }
+    if (prof_) prof_->mark("mri_gram_setup", st);
+    pl.body = [=](int par, cudaStream_t s) {
+      GramImage g{};
+      g.W = W_;
+      g.H = H_;
+      g.src = ptrs(p0 ^ par ^ 1);  // this iteration's p, q
+      g.dst = ptrs(p0 ^ par);      // the next one's
+      g.dst.ub = g.src.ub;         // u-bar and v-bar of the last iteration join its p, q
+      g.dst.vbx = g.src.vbx;
+      g.dst.vby = g.src.vby;
+      auto primal = [&](ImgPtrs& q, int set) {
+        q.u = raw_field(F_U, set);
+        q.vx = raw_field(F_VX, set);
+        q.vy = raw_field(F_VY, set);
+      };
+      primal(g.src, par);
+      primal(g.dst, par ^ 1);
+      g.U = U + 2 * N * par;
+      g.Unext = U + 2 * N * (par ^ 1);
+      g.part = part;
+      g.groups = rows.groups;
+      g.b = b;
+      g.z0 = r_zero ? nullptr : z0;
+      g.table = table;
+      g.header = header;
+      g.par = par;
+      g.tau = tau;
+      g.sigma = sigma;
+      g.lambda = lambda;
+      g.k = k;
+      launch_gram_rows(rows, g.U, part, s);
+      if (prof_) prof_->mark("mri_gram_rows", s);
+      launch_gram_image(is_tgv, g, s);
+      if (prof_) prof_->mark(is_tgv ? "mri_gram_image_tgv" : "mri_gram_image_tv", s);
+    };
+    pl.post = [=](cudaStream_t s) {
+      if (n & 1)  // the results lie in the second copies
+        for (int f : {(int)F_U, (int)F_VX, (int)F_VY})
+          if (f == F_U || is_tgv)
+            PDT_CUDA_CHECK(cudaMemcpyAsync(raw_field(f, 0), raw_field(f, 1), plane, cudaMemcpyDeviceToDevice, s));
+      hk->dual_from_image(U + 2 * N * ((n - 1) & 1), r_.as<float2>(), fc_.as<float2>(), c, d, s);
+      if (prof_) prof_->mark("mri_gram_dual", s);
+    };
+    pl.key = graph_key({(uintptr_t)img_.p, (uintptr_t)gram_.p, (uintptr_t)alpha_.p, (uintptr_t)alpha_.bytes,
+                        (uintptr_t)op_.get(), (uintptr_t)op_->generation(), (uintptr_t)W_, (uintptr_t)H_, (uintptr_t)p0,
+                        (uintptr_t)is_tgv, (uintptr_t)r_zero, fbits(lambda), fbits(tau), fbits(sigma),
+                        (uintptr_t)version_, (uintptr_t)1});
   }
 
   void ensure_fc(SolverHooks* hk, cudaStream_t st) {
@@ -956,6 +1055,7 @@ class OptImpl {
 
   static constexpr int kGraphIters = 20;
   static constexpr size_t kAlphaHeader = 64;
+  static constexpr unsigned kGramMinIters = 8;
 
   pdt_opt_kind kind_;
   bool cplx_;
@@ -967,7 +1067,7 @@ class OptImpl {
   Dims usize_;
   int W_ = 0, H_ = 0;
   int parity_ = 0;
-  DevBuf img_, r_, fc_, khr_, alpha_;
+  DevBuf img_, r_, fc_, khr_, alpha_, gram_;
   std::vector<float> alpha_host_;
   bool r_reset_ = true, fc_valid_ = false;
   uint64_t op_gen_ = 0;
@@ -1072,6 +1172,7 @@ class BatchImpl {
     fork_join(st, [&](size_t i, cudaStream_t w) {
       for (int it = full * kBatchIters; it < plans[i].n; ++it) plans[i].body(it & 1, w);
       for (int t = 0; t < plans[i].tail; ++t) plans[i].tail_body((plans[i].n + t) & 1, w);
+      if (plans[i].post) plans[i].post(w);
     });
     for (size_t i = 0; i < opts_.size(); ++i) opts_[i]->finish(plans[i]);
   }

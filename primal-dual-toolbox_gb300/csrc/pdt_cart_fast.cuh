@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(32 * WPB) fl_cols(CartDev d, int mode, const f
   const int kb = M * lane_brev<L>(t);
   const float* mrow = d.maskc + (size_t)s * Hf;
   float2 v[M];
-  if (mode == COL_SOLVE || mode == COL_FWD_DENSE) {
+  if (mode == COL_SOLVE || mode == COL_FWD_DENSE || mode == COL_DUAL) {
 #pragma unroll
     for (int j = 0; j < M; ++j) {
       int yf = t + L * j - d.mxH;
@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(32 * WPB) fl_cols(CartDev d, int mode, const f
       for (int q = 0; q < CH; ++q) {
         if (k0 + q < M) {
           const float2 kv = v[k0 + q] * (d.scale * m[q]);
-          rv[q] = (rv[q] + sigma * (kv - fv[q])) / (1.0f + sigma * lambda);
+          rv[q] = mode == COL_DUAL ? lambda * rv[q] + (kv - sigma * fv[q])
+                                   : (rv[q] + sigma * (kv - fv[q])) / (1.0f + sigma * lambda);
           v[k0 + q] = rv[q] * m[q];
         }
       }
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(32 * WPB) fl_cols(CartDev d, int mode, const f
           if (k0 + q < M) rcol[(k0 + q) * L + t] = rv[q];
       }
     }
+    if (mode == COL_DUAL) return;
   } else {
 #pragma unroll
     for (int k1 = 0; k1 < M; ++k1) {
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(32 * WPB) fl_cols64(CartDev d, int mode, const
   const int kb = M * (int)(__brev((unsigned)t) >> 26);
   const float* mrow = d.maskc + (size_t)s * Hf;
   float2 v[M];
-  if (mode == COL_SOLVE || mode == COL_FWD_DENSE) {
+  if (mode == COL_SOLVE || mode == COL_FWD_DENSE || mode == COL_DUAL) {
 #pragma unroll
     for (int j = 0; j < M; ++j) {
       if ((ZM >> j) & 1) {
@@ -246,13 +248,15 @@ __global__ void __launch_bounds__(32 * WPB) fl_cols64(CartDev d, int mode, const
 #pragma unroll
     for (int k1 = 0; k1 < M; ++k1) {
       const float2 kv = v[k1] * (d.scale * m[k1]);
-      rv[k1] = (rv[k1] + sigma * (kv - fv[k1])) / (1.0f + sigma * lambda);
+      rv[k1] = mode == COL_DUAL ? lambda * rv[k1] + (kv - sigma * fv[k1])
+                                : (rv[k1] + sigma * (kv - fv[k1])) / (1.0f + sigma * lambda);
       v[k1] = rv[k1] * m[k1];
     }
     if (ok) {
 #pragma unroll
       for (int k1 = 0; k1 < M; ++k1) rcol[k1 * L + t] = rv[k1];
     }
+    if (mode == COL_DUAL) return;
   } else {
 #pragma unroll
     for (int k1 = 0; k1 < M; ++k1) {

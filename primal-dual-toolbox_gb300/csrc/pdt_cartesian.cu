@@ -60,7 +60,8 @@ struct CartDev {
   int tc_yb;  // tensor-core row passes: image rows per 128-row tile (the tile holds them for every coil)
 };
 
-enum ColMode { COL_SOLVE = 0, COL_FWD_DENSE = 1, COL_ADJ_DENSE = 2, COL_ADJ_COMPACT = 3 };
+// COL_DUAL: r <- lambda r + K u - sigma f (no inverse transform)
+enum ColMode { COL_SOLVE = 0, COL_FWD_DENSE = 1, COL_ADJ_DENSE = 2, COL_ADJ_COMPACT = 3, COL_DUAL = 4 };
 
 __device__ __forceinline__ int imod(int a, int n) {
   a %= n;
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(kThreads) cols_kernel(CartDev d, int mode, con
 
   float2* Y;  // inverse-FFT input buffer
   float2* Yo;
-  if (mode == COL_SOLVE || mode == COL_FWD_DENSE) {
+  if (mode == COL_SOLVE || mode == COL_FWD_DENSE || mode == COL_DUAL) {
     for (int i = threadIdx.x; i < ncb * Hf; i += blockDim.x) {
       const int cb = i / Hf, j = i - cb * Hf;
       const int yf = imod(j - d.mxH, Hf);  // image row that lands in FFT slot j after ifftshift
@@ -138,13 +139,17 @@ __global__ void __launch_bounds__(kThreads) cols_kernel(CartDev d, int mode, con
         kout[((size_t)c * Hf + ypos) * d.W + d.col_x[s]] = k;
       } else {
         const size_t o = ((size_t)c * d.ns + s) * Hf + ypos;
+        if (mode == COL_DUAL) {
+          r[o] = lambda * r[o] + (k - sigma * fc[o]);
+          continue;
+        }
         // addWeighted(tmp, 1, f, -1) then TGV_prox_r_kernel (tgvmrioptimizer.cu:167-174)
         const float2 rn = (r[o] + sigma * (k - fc[o])) / (1.0f + sigma * lambda);
         r[o] = rn;
         Y[cb * d.ldH + imod(ypos + d.mxH, Hf)] = rn * m;  // preifft_kernel
       }
     }
-    if (mode == COL_FWD_DENSE) return;
+    if (mode == COL_FWD_DENSE || mode == COL_DUAL) return;
     Yo = X;
   } else {
     Y = A;
@@ -283,6 +288,16 @@ class CartesianOp : public OpImpl, public SolverHooks {
     return constant(0, PDT_C64, 3).size;
   }
   SolverHooks* hooks() override { return this; }
+  const GramRows* line_gram() override {
+    prepare();
+    return gram_.len.n ? &gram_ : nullptr;
+  }
+  void dual_from_image(const float2* U, float2* r, const float2* fc, float c, float d, cudaStream_t st) override {
+    prepare();
+    float2* t = scratch_.as<float2>();
+    launch_rows_fwd(U, t, nullptr, st);
+    launch_cols(COL_DUAL, t, nullptr, r, fc, nullptr, nullptr, c, d, st);
+  }
   void check_device_errors() override {
     if (const int e = take_tc_error()) {
       char code[16];
@@ -324,6 +339,9 @@ class CartesianOp : public OpImpl, public SolverHooks {
     if (tune_.tca && dev_.ns > 0 && fuse_dual_ && dual_rows() > 0)
       os << " solver_dual=adjoint_launch(" << dual_rows() * ((2 * dev_.W + tc_adj_nb(tune_.nr) - 1) / tc_adj_nb(tune_.nr))
          << "_blocks)";
+    if (gram_.len.n)
+      os << " solver=line_gram(" << gram_.len.P << "x" << gram_.len.Q << (gram_.len.n == dev_.W ? "" : ",padded") << ",coil_sums="
+         << gram_.groups << ")";
     if (frow_.ok())  // what a batched solve runs (tca(), tcf(), groups_run())
       os << " in_batch=lane_fft_rows(batch_adj_groups=" << std::min(G_, batch_groups())
          << (tune_.cluster ? ",cluster" : ",partials") << ")";
@@ -401,7 +419,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
       launch_rows_adj(t, khr, groups_run(), st);
     if (mk) mk->mark("cart_rows_adj", st);
   }
-  void adjoint_compact(const float2* fc, float2* img, cudaStream_t st) override {
+  void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool exact_rows) override {
     prepare();
     if (dev_.ns == 0) {
       launch_fill_zero(img, sizeof(float2) * (size_t)dev_.Hi * dev_.W, st);
@@ -409,7 +427,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
     }
     float2* t = scratch_.as<float2>();
     launch_cols(COL_ADJ_COMPACT, nullptr, t, nullptr, fc, nullptr, nullptr, 0.f, 0.f, st);
-    if (tca())
+    if (tca() && !exact_rows)
       launch_tc_rows_adj(t, img, st);
     else
       launch_rows_adj(t, img, 1, st);
@@ -792,7 +810,39 @@ class CartesianOp : public OpImpl, public SolverHooks {
     dev_ = d;
     autotune();
     dev_ = d;
+    prepare_gram(mask, col_x);
     prepared_ = true;
+  }
+
+  // The solvers' row operator (pdt_gram.h) where every sampled column of the mask is constant along the
+  // readout. A pinned tuning pins the three-pass round as well.
+  void prepare_gram(const float* mask, const std::vector<int>& col_x) {
+    gram_ = GramRows();
+    const char* pin = std::getenv("PDT_CARTESIAN_TUNE");
+    if (dev_.ns == 0 || (pin && *pin)) return;
+    for (int y = 1; y < dev_.Hf; ++y)
+      for (int x : col_x)
+        if (!(mask[(size_t)y * dev_.W + x] == mask[x])) return;
+    const GramLength len = gram_length(dev_.W);
+    if (!len.n) return;
+    std::vector<float> m2(dev_.W, 0.f), spec;
+    for (int x : col_x) m2[(x + dev_.W - dev_.oxW) % dev_.W] = mask[x] * mask[x];  // DFT index of column x
+    std::vector<float2> tw;
+    gram_tables(dev_.W, len, m2, tw, spec);
+    gram_tab_.ensure(len.n * (sizeof(float2) + sizeof(float)));
+    std::vector<char> host(gram_tab_.bytes);
+    std::memcpy(host.data(), tw.data(), sizeof(float2) * len.n);
+    std::memcpy(host.data() + sizeof(float2) * len.n, spec.data(), sizeof(float) * len.n);
+    PDT_CUDA_CHECK(cudaMemcpy(gram_tab_.p, host.data(), host.size(), cudaMemcpyHostToDevice));
+    gram_.W = dev_.W;
+    gram_.H = dev_.Hi;
+    gram_.C = dev_.C;
+    gram_.sens = dev_.sens ? dev_.sens + (size_t)dev_.y0 * dev_.W : nullptr;
+    gram_.coil_stride = (size_t)dev_.Hf * dev_.W;
+    gram_.len = len;
+    gram_.tw = gram_tab_.as<float2>();
+    gram_.spec = reinterpret_cast<const float*>(gram_tab_.as<float2>() + len.n);
+    gram_.groups = gram_groups(len, dev_.Hi, dev_.C, g_num_sms);
   }
 
   // Times the candidate launch shapes of the lane-FFT kernels on scratch buffers (CUDA events, a
@@ -994,7 +1044,8 @@ class CartesianOp : public OpImpl, public SolverHooks {
   int tcb_nb_ = 0;         // range size the adjoint DFT tiles in tcb_ were built for
   bool tcf_built_ = false;  // forward DFT tiles in tcf_tiles_
   int G_ = 1;
-  DevBuf tables_, scratch_, tc_err_, tcb_, tcf_tiles_;
+  GramRows gram_;
+  DevBuf tables_, scratch_, tc_err_, tcb_, tcf_tiles_, gram_tab_;
 };
 
 std::shared_ptr<OpImpl> make_cartesian_operator(pdt_op_kind kind) { return std::make_shared<CartesianOp>(kind); }

@@ -1,0 +1,78 @@
+// pdt_gram.h -- the iterations of the with-operator solvers for masks of whole phase-encode lines.
+//
+// When every sampled column of the mask is constant along the readout, the readout transforms of K and K^H
+// cancel and K^H K acts on each image row by itself:
+//   (K^H K u)(y, .) = sum_c conj(s_c) . G (s_c . u)(y, .),   G = (1 / W) IDFT diag(m^2) DFT along the row,
+// and the k-space dual of r <- (r + sigma (K ubar - f)) / (1 + sigma lambda) stays in the span
+//   r_n = K U_n - c_n f + d_n r_0,   U <- U + k (ubar - lambda U),  k = sigma / (1 + sigma lambda),
+//   c <- c + k (1 - lambda c) from 0,   d <- d - k lambda d from 1,
+// so that K^H r_n = K^H K U_n - c_n K^H f + d_n K^H r_0 needs one image U, two fixed images and the row
+// operator G: no k-space array and no transform along the readout inside an iteration. U is carried with a
+// compensation term (the rounding errors of its updates, as in Kahan's summation): without it an update
+// below half a unit in the last place of U is lost, and U stops up to (1 + sigma lambda) / (2 sigma lambda)
+// units away from its limit, which K^H K passes on to u in every iteration.
+//
+// One iteration is two launches: launch_gram_rows (K^H K U in coil-group partial sums) and
+// launch_gram_image (primal update, then the next iteration's dual update and U).
+#pragma once
+
+#include <cstddef>
+#include <vector>
+
+#include "pdt_internal.h"
+
+namespace pdt {
+
+// One compiled transform length n = P Q (P values per thread, then Q).
+struct GramLength {
+  int n, P, Q;
+};
+
+// What an operator with a line mask hands to the solvers.
+struct GramRows {
+  int W = 0, H = 0, C = 0;        // image and coils
+  const float2* sens = nullptr;   // coil 0, image row 0, or null (one coil without a map)
+  size_t coil_stride = 0;         // elements between coils
+  GramLength len{0, 0, 0};
+  const float2* tw = nullptr;     // [Q][P] exp(-2 pi i t k1 / n)
+  const float* spec = nullptr;    // [n] spectrum of G in the natural order, scaled for an unscaled inverse
+  int groups = 1;                 // coil-group partial sums of K^H K U
+};
+
+// The compiled length for rows of W: W itself, or the smallest one that holds the linear convolution
+// (n >= 2 W - 1), in which G is embedded as a Toeplitz operator. n = 0: none.
+GramLength gram_length(int W);
+
+// Coil groups for an H-row image on a GPU of `sms` multiprocessors.
+int gram_groups(const GramLength& len, int H, int C, int sms);
+
+// Host tables (tw: n values, spec: n values) of the row operator. m2[k]: squared mask value at the DFT
+// index k of a row (0 where not sampled).
+void gram_tables(int W, const GramLength& len, const std::vector<float>& m2, std::vector<float2>& tw,
+                 std::vector<float>& spec);
+
+struct GramImage {
+  int W, H;
+  ImgPtrs src;           // u, v and the p, q of this iteration
+  ImgPtrs dst;           // new u, v; ubar, vbar (last iteration only); p, q of the next iteration
+  const float2* U;       // this iteration's U, then its compensation (W x H each)
+  float2* Unext;
+  const float2* part;    // `groups` partial sums of K^H K U, W x H each
+  int groups;
+  const float2* b;       // K^H f
+  const float2* z0;      // K^H r_0, or null when r_0 = 0
+  const float4* table;   // per iteration {alpha0, alpha1, c, d}
+  int* header;           // [1] table length, [2] non-finite flag, [4], [5] iteration counters (see par)
+  int par;               // this iteration's counter is header[4 + par]; it sets header[4 + (par ^ 1)]
+  float tau, sigma, lambda, k;
+};
+
+// part[g] <- sum of conj(s_c) . G (s_c . U) over the coils of group g.
+void launch_gram_rows(const GramRows& g, const float2* U, float2* part, cudaStream_t st);
+// u, v <- the primal update from part; then, unless this is the table's last iteration, p, q and U of the
+// next one (the last iteration stores ubar and vbar instead). Raises header[2] on a non-finite u or v.
+void launch_gram_image(bool tgv, const GramImage& s, cudaStream_t st);
+// U <- k ubar, compensation 0: the first iteration's U, from U_0 = 0.
+void launch_gram_start(int W, int H, const float2* ubar, float k, float2* U, cudaStream_t st);
+
+}  // namespace pdt

@@ -6,6 +6,7 @@
 #include <string>
 #include <vector>
 
+#include "pdt_gram.h"
 #include "pdt_internal.h"
 
 namespace pdt {
@@ -50,8 +51,14 @@ struct SolverHooks {
   virtual void set_concurrent(bool on) {}
   virtual int groups() = 0;
   virtual long long group_stride() = 0;
+  // The row operator of a line mask (pdt_gram.h), or null where the solvers run round().
+  virtual const GramRows* line_gram() { return nullptr; }
+  // r <- d r + K U - c f in the compact layout (the k-space dual after iterations with line_gram()).
+  virtual void dual_from_image(const float2* U, float2* r, const float2* fc, float c, float d, cudaStream_t st) {}
   // img <- K^H f from the compact layout (the solver's initial u0 = A^T f).
-  virtual void adjoint_compact(const float2* fc, float2* img, cudaStream_t st) = 0;
+  // `exact_rows`: with row transforms whose error is that of FP32 rounding also where another kernel (TF32
+  // triples, about 1e-6 relative) is faster.
+  virtual void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool exact_rows = false) = 0;
 };
 
 class OpImpl {

@@ -399,7 +399,7 @@ class RadialOp : public OpImpl, public SolverHooks {
     if (mk) mk->mark("rad_degrid_prox", st);
     adjoint_from_weighted(svals_.as<float2>(), khr, G_, st, mk);
   }
-  void adjoint_compact(const float2* fc, float2* img, cudaStream_t st) override {
+  void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool) override {
     prepare();
     launch_weight(fc, st);
     adjoint_from_weighted(svals_.as<float2>(), img, 1, st, nullptr);
