@@ -85,19 +85,14 @@ struct DualStep {
   int tgv;  // 1: TGV (p and q), 0: TV (p only)
 };
 
-// Fused TvOptimizer iteration (tgv_kernels.cuh:294-324 then 568-605): reads u, u-bar and p from `in`,
-// writes them to `out`.
-void launch_tv_step(bool complex_, int W, int H, const ImgPtrs& in, const ImgPtrs& out, const void* f, float tau,
-                    float sigma, float lambda, cudaStream_t st);
-// kTvStepsPerLaunch TvOptimizer iterations in one launch (temporal blocking in shared memory); same
-// arithmetic per pixel as launch_tv_step, state read from `in` and written to `out`.
-constexpr int kTvStepsPerLaunch = 4;
-void launch_tv_multi_step(bool complex_, int W, int H, const ImgPtrs& in, const ImgPtrs& out, const void* f,
-                          float tau, float sigma, float lambda, cudaStream_t st);
-
-// Fused TgvOptimizer iteration, primal first (tgvoptimizer.cu:117-137): every field ping-pongs.
-void launch_tgv_denoise_step(bool complex_, int W, int H, const ImgPtrs& in, const ImgPtrs& out, const void* f,
-                             float tau, float sigma, float lambda, float alpha0, float alpha1, cudaStream_t st);
+// TvOptimizer / TgvOptimizer, `steps` iterations in one launch (pdt_denoise.cu): state from `in` to `out`; TGV's u-bar
+// and v-bar, which no iteration reads, only with store_bar.
+// denoise_steps: iterations per launch for a solve of `iters` on this image (iters itself where one block holds the
+// image, launched with halo 0; else the halo) and the region that launch_denoise is then given.
+int denoise_steps(bool complex_, bool tgv, int W, int H, int iters, int* region);
+void launch_denoise(bool complex_, bool tgv, int W, int H, const ImgPtrs& in, const ImgPtrs& out, const void* f, float tau,
+                    float sigma, float lambda, float alpha0, float alpha1, int region, int halo, int steps,
+                    bool store_bar, cudaStream_t st);
 
 // Image side of one TgvMri / TgvWithOp / TvWithOp iteration (tgvmrioptimizer.cu:177-197).
 // Dual: p, q from u-bar, v-bar of `in` into `out`; alpha_tab[2k], alpha_tab[2k+1] = alpha0, alpha1 of
