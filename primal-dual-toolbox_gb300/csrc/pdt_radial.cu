@@ -10,15 +10,14 @@
 // continuous Fourier transform. Trajectory {Ns, 2} is planar (k0 for all samples, then k1; k0 pairs with
 // image x); dcf {Ns, 1}; coil maps {N, N, C}.
 //
-// Kernels (all FFTs are the batched shared-memory FFT of pdt_device.cuh over the G-point axes):
-//   rad_rows_fwd   image rows . sens_c / deap  -> zero-padded FFT along x   -> T[c][gx][image row]
-//   rad_cols       FFT along y of each grid column (input on the N image rows) -> F[c][gx][gy]
+// The grid F[gy][gx][c], the samples' k-space arrays [j][c] (the solvers' compact layout) and, with compiled grid
+// lengths, the half-transformed rows have the coils innermost: gridding and degridding move all coils of a cell or
+// sample as one run, a thread per (cell, coil) or (sample, coil).
+//   rl_rows_fwd, rl_cols, rl_rows_inv   transform passes for compiled grid lengths (pdt_rad_fast.cuh)
+//   rad_rows_fwd, rad_cols, ...         the same for other lengths (batched shared-memory FFT of pdt_device.cuh)
 //   rad_degrid     per sample: 9 (W^2) taps of F, dcf weight; solver mode adds the k-space dual prox
-//   rad_grid       gridding as a gather: one thread per grid cell walks the samples whose footprint covers
-//                  the cell, in sample order, with their tap weights (lists built at set-up) --
-//                  deterministic, no atomics
-//   rad_cols_inv   IFFT along y of each grid column, keep the N image rows
-//   rad_rows_inv   IFFT along x, crop, / deap, conj(sens_c) . and the coil sum
+//   rad_grid       gridding as a gather: each grid cell walks the samples whose footprint covers it, in sample
+//                  order, with their tap weights (lists built at set-up) -- deterministic, no atomics
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -36,7 +35,7 @@ constexpr int kRT = 256;   // threads per block
 constexpr int kMaxKw = 8;  // largest supported kernel width
 constexpr int kRR = 4;     // rows per block in the row passes
 constexpr int kRC = 4;     // columns per block in the column passes
-constexpr int kHeavy = 12; // gridding: cells with longer sample lists get a warp each
+constexpr int kHeavy = 24; // gridding: cells with longer sample lists get a block each
 
 struct RadDev {
   int N, G, C, Ns, kw;
@@ -48,10 +47,10 @@ struct RadDev {
   const float* w;       // [Ns] density compensation
   const int* g0;        // [2*Ns] gx0, gy0 (may be negative; wrap mod G)
   const float* wt;      // [Ns][2][kw] tap weights (x then y)
-  const int* cell_ptr;  // [G*G+1] per grid cell gx * G + gy: range of its entries
+  const int* cell_ptr;  // [G*G+1] per grid cell gy * G + gx: range of its entries
   const int* cell_idx;  // samples whose footprint covers the cell, ascending
   const float* cell_w;  // their tap weights wx * wy
-  const int* heavy;     // cells with more than kHeavy entries (gridded one warp per cell)
+  const int* heavy;     // cells with more than kHeavy entries (gridded one block per cell)
   int n_heavy;
   const float2* tw;     // [G]
   FftPlan plan;
@@ -106,157 +105,137 @@ __global__ void __launch_bounds__(kRT) rad_cols(RadDev d, const float2* __restri
   __syncthreads();
   const float2* X = smem_fft(A, B, ncb, d.ldG, d.plan, tw, false);
   for (int i = threadIdx.x; i < ncb * d.G; i += blockDim.x) {
-    const int cb = i / d.G, gy = i - cb * d.G;
-    F[((size_t)c * d.G + gx0 + cb) * d.G + gy] = X[cb * d.ldG + gy];
+    const int gy = i / ncb, cb = i - gy * ncb;
+    F[((size_t)gy * d.G + gx0 + cb) * d.C + c] = X[cb * d.ldG + gy];
   }
 }
 
-// Degridding. mode 0: kout[c][j] = A u. mode 1 (solver): r <- (r + sigma (A u - f)) / (1 + sigma lambda),
-// s[j][c] = w_j r (the weighted values the adjoint grids, sample-major). blockIdx.y selects a chunk of MAXC
-// coils, fully unrolled, so that a sample's tap loads of the chunk are all in flight at once; KW > 0 fixes
-// the kernel width at compile time so that the taps unroll too (KW = 0: d.kw at run time).
-template <int MAXC, int KW>
+// Degridding, a thread per (sample, coil), coils fastest. mode 0: kout[c][j] = A u (the user's layout). mode 1
+// (solver): r <- (r + sigma (A u - f)) / (1 + sigma lambda), s[j][c] = w_j r (the weighted values the adjoint
+// grids). KW > 0 fixes the kernel width at compile time so that the taps unroll (KW = 0: d.kw at run time). Bound by L2:
+// KW^2 runs of C values a sample (12 coils, 32768 samples: 28 MB).
+template <int KW>
 __global__ void __launch_bounds__(kRT) rad_degrid(RadDev d, int mode, const float2* __restrict__ F,
                                                   float2* __restrict__ kout, float2* __restrict__ r,
                                                   const float2* __restrict__ f, float2* __restrict__ s,
                                                   float sigma, float lambda) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= d.Ns) return;
+  const unsigned i = blockIdx.x * kRT + threadIdx.x;
+  const unsigned j = i / (unsigned)d.C, c = i - j * (unsigned)d.C;
+  const bool ok = j < (unsigned)d.Ns;
   static_assert(KW >= 0 && KW <= kMaxKw, "kernel width");
   const int kw = KW > 0 ? KW : d.kw;
   float wx[kMaxKw], wy[kMaxKw];
   int gxs[kMaxKw], gys[kMaxKw];
+  float wj = 0.f;
+  if (ok) {
 #pragma unroll
-  for (int t = 0; t < kw; ++t) {
-    wx[t] = d.wt[((size_t)j * 2 + 0) * kw + t];
-    wy[t] = d.wt[((size_t)j * 2 + 1) * kw + t];
-    gxs[t] = wrapG(d.g0[2 * j] + t, d.G);
-    gys[t] = wrapG(d.g0[2 * j + 1] + t, d.G);
+    for (int t = 0; t < kw; ++t) {
+      wx[t] = d.wt[((size_t)j * 2 + 0) * kw + t];
+      wy[t] = d.wt[((size_t)j * 2 + 1) * kw + t];
+      gxs[t] = wrapG(d.g0[2 * j] + t, d.G);
+      gys[t] = wrapG(d.g0[2 * j + 1] + t, d.G) * d.G;
+    }
+    wj = d.w[j];
   }
-  const float wj = d.w[j];
-  const size_t plane = (size_t)d.G * d.G;
-  {
-    const int cbase = blockIdx.y * MAXC;
-    const int nc = min(MAXC, d.C - cbase);
-    float2 a[MAXC];
+  pdl_wait();  // F comes from the previous kernel
+  pdl_trigger();
+  if (!ok) return;
+  const float2 ro = mode ? r[i] : c2(0.f, 0.f), fo = mode ? f[i] : c2(0.f, 0.f);
+  float2 a = c2(0.f, 0.f);
 #pragma unroll
-    for (int c = 0; c < MAXC; ++c) a[c] = c2(0.f, 0.f);
+  for (int tx = 0; tx < kw; ++tx) {
+    float2 col = c2(0.f, 0.f);
 #pragma unroll
-    for (int tx = 0; tx < kw; ++tx) {
-      float2 col[MAXC];
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c) col[c] = c2(0.f, 0.f);
-#pragma unroll
-      for (int ty = 0; ty < kw; ++ty) {
-        const float2* Fp = F + (size_t)cbase * plane + (size_t)gxs[tx] * d.G + gys[ty];
-#pragma unroll
-        for (int c = 0; c < MAXC; ++c)
-          if (c < nc) col[c] += Fp[(size_t)c * plane] * wy[ty];
-      }
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c) a[c] += col[c] * wx[tx];
-    }
-#pragma unroll
-    for (int c = 0; c < MAXC; ++c) {
-      if (c >= nc) break;
-      const float2 av = a[c] * wj;
-      const size_t o = (size_t)(cbase + c) * d.Ns + j;
-      if (mode == 0) {
-        kout[o] = av;
-      } else {
-        const float2 rn = (r[o] + sigma * (av - f[o])) / (1.0f + sigma * lambda);
-        r[o] = rn;
-        s[(size_t)j * d.C + cbase + c] = rn * wj;  // sample-major for the gridding gather
-      }
-    }
+    for (int ty = 0; ty < kw; ++ty) col += F[(size_t)(gys[ty] + gxs[tx]) * d.C + c] * wy[ty];
+    a += col * wx[tx];
+  }
+  const float2 av = a * wj;
+  if (mode == 0) {
+    kout[(size_t)c * d.Ns + j] = av;
+  } else {
+    const float2 rn = (ro + sigma * (av - fo)) / (1.0f + sigma * lambda);
+    r[i] = rn;
+    s[i] = rn * wj;
   }
 }
 
-// s[j][c] = w_j k[c][j] (adjoint input weighting for a dense k-space, sample-major).
-__global__ void rad_weight(RadDev d, const float2* __restrict__ k, float2* __restrict__ s) {
+// s[j][c] = w_j k: of the user's layout k[c][j] (dense) or the compact one k[j][c].
+__global__ void rad_weight(RadDev d, const float2* __restrict__ k, int dense, float2* __restrict__ s) {
   const size_t n = (size_t)d.C * d.Ns;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t c = i / d.Ns, j = i - c * d.Ns;
-    s[j * d.C + c] = k[i] * d.w[j];
+    const size_t j = i / d.C, c = i - j * d.C;
+    s[i] = k[dense ? c * d.Ns + j : i] * d.w[j];
   }
 }
 
-// Gridding as a gather: H[c][gx][gy] = sum_j s[j][c] wx[gx - gx0_j] wy[gy - gy0_j] over the samples j whose
-// footprint covers the cell (lists built at set-up, entries in sample order). One launch, two kinds of
-// block: the first heavy_blocks blocks give each of the cells near k = 0 (more than kHeavy entries) a
-// warp, lane l taking entries l, l + 32, ... and an xor-butterfly sum (every lane ends with the same,
-// run-to-run identical value); the others give every remaining cell a thread that walks its list in
-// order, four entries at a time so that many loads are in flight. A sample's coil values are contiguous.
-template <int MAXC>
-__global__ void __launch_bounds__(kRT) rad_grid(RadDev d, const float2* __restrict__ s, float2* __restrict__ H,
-                                                int heavy_blocks) {
-  const size_t ncell = (size_t)d.G * d.G;
-  if ((int)blockIdx.x < heavy_blocks) {
-    const int wi = blockIdx.x * (kRT / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (wi >= d.n_heavy) return;  // uniform per warp
-    const int cell = d.heavy[wi];
+// compact[j][c] <- dense[c][j], or back.
+__global__ void rad_transpose(RadDev d, const float2* __restrict__ in, float2* __restrict__ out, int to_dense) {
+  const size_t n = (size_t)d.C * d.Ns;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t j = i / d.C, c = i - j * d.C, o = c * d.Ns + j;
+    if (to_dense)
+      out[o] = in[i];
+    else
+      out[i] = in[o];
+  }
+}
+
+// Gridding as a gather: H[gy][gx][c] = sum_j s[j][c] wx[gx - gx0_j] wy[gy - gy0_j] over the samples j whose
+// footprint covers the cell (lists built at set-up, entries in sample order). One launch, two kinds of block:
+// the first n_heavy blocks take a cell near k = 0 (more than kHeavy entries) each, thread (slot, coil) summing
+// every slots-th entry and the slots added in order; the others give each (cell, coil) a thread that walks the
+// cell's list in order, four entries at a time so that many loads are in flight. A warp's loads of s are runs of C
+// values (a thread per cell and all coils, as before, touched 32 runs a load: 20 us instead of 6 for 12 coils on 384^2).
+__global__ void __launch_bounds__(kRT) rad_grid(RadDev d, const float2* __restrict__ s, float2* __restrict__ H) {
+  const int C = d.C;
+  if ((int)blockIdx.x < d.n_heavy) {
+    __shared__ float2 part[kRT];
+    const int cell = d.heavy[blockIdx.x];
     const int beg = d.cell_ptr[cell], end = d.cell_ptr[cell + 1];
-    for (int cbase = 0; cbase < d.C; cbase += MAXC) {
-      const int nc = min(MAXC, d.C - cbase);
-      float2 acc[MAXC];
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c) acc[c] = c2(0.f, 0.f);
-      for (int e = beg + lane; e < end; e += 32) {
-        const float2* sj = s + (size_t)d.cell_idx[e] * d.C + cbase;
-        const float wgt = d.cell_w[e];
-#pragma unroll
-        for (int c = 0; c < MAXC; ++c)
-          if (c < nc) acc[c] += sj[c] * wgt;
+    const int cw = min(C, kRT), slots = kRT / cw, c0 = threadIdx.x % cw, slot = threadIdx.x / cw;
+    pdl_wait();  // s comes from the previous kernel
+    pdl_trigger();
+    for (int cb = 0; cb < C; cb += cw) {
+      const int c = cb + c0;
+      float2 acc = c2(0.f, 0.f);
+      if (slot < slots && c < C) {
+#pragma unroll 4
+        for (int e = beg + slot; e < end; e += slots) acc += s[(size_t)d.cell_idx[e] * C + c] * d.cell_w[e];
       }
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c) {
-        if (c < nc) {
-          for (int o = 16; o > 0; o >>= 1) {
-            acc[c].x += __shfl_xor_sync(0xffffffffu, acc[c].x, o);
-            acc[c].y += __shfl_xor_sync(0xffffffffu, acc[c].y, o);
-          }
-          if (lane == 0) H[(size_t)(cbase + c) * ncell + cell] = acc[c];
-        }
+      part[threadIdx.x] = acc;
+      __syncthreads();
+      if (slot == 0 && c < C) {
+        for (int q = 1; q < slots; ++q) acc += part[q * cw + c0];
+        H[(size_t)cell * C + c] = acc;
       }
+      __syncthreads();
     }
     return;
   }
-  const size_t cell = (blockIdx.x - heavy_blocks) * (size_t)blockDim.x + threadIdx.x;
-  if (cell >= ncell) return;
-  const int beg = d.cell_ptr[cell], end = d.cell_ptr[cell + 1];
-  if (end - beg > kHeavy) return;  // a heavy block's warp grids it
-  for (int cbase = 0; cbase < d.C; cbase += MAXC) {
-    const int nc = min(MAXC, d.C - cbase);
-    float2 acc[MAXC];
+  const size_t i = (blockIdx.x - d.n_heavy) * (size_t)kRT + threadIdx.x;
+  const unsigned cell = (unsigned)(i / (unsigned)C);
+  const bool ok = cell < (unsigned)(d.G * d.G);
+  const int beg = ok ? d.cell_ptr[cell] : 0, end = ok ? d.cell_ptr[cell + 1] : 0;
+  const float2* sc = s + (i - (size_t)cell * C);
+  pdl_wait();
+  pdl_trigger();
+  if (!ok || end - beg > kHeavy) return;  // a block of its own grids it
+  float2 acc = c2(0.f, 0.f);
+  for (int e = beg; e < end; e += 4) {
+    const int m = end - e;  // entries e .. e + min(m, 4) - 1 are this cell's
+    float2 v[4];
+    float w[4];
 #pragma unroll
-    for (int c = 0; c < MAXC; ++c) acc[c] = c2(0.f, 0.f);
-    // four entries at a time, the last group predicated (most cells have fewer than four), so that a
-    // group's index and weight loads, then its sample loads, are each in flight together
-    for (int e = beg; e < end; e += 4) {
-      const int m = end - e;  // entries e .. e + min(m, 4) - 1 are this cell's
-      const float2* sp[4];
-      float w[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        sp[k] = s + (size_t)(k < m ? d.cell_idx[e + k] : 0) * d.C + cbase;
-        w[k] = k < m ? d.cell_w[e + k] : 0.f;
-      }
-#pragma unroll
-      for (int c = 0; c < MAXC; ++c)
-        if (c < nc) {  // loads only for this cell's entries, added in entry order as one at a time
-          const float2 z = c2(0.f, 0.f);
-          const float2 a0 = sp[0][c], a1 = m > 1 ? sp[1][c] : z, a2 = m > 2 ? sp[2][c] : z,
-                       a3 = m > 3 ? sp[3][c] : z;
-          acc[c] += a0 * w[0];
-          if (m > 1) acc[c] += a1 * w[1];
-          if (m > 2) acc[c] += a2 * w[2];
-          if (m > 3) acc[c] += a3 * w[3];
-        }
+    for (int k = 0; k < 4; ++k) {
+      w[k] = k < m ? d.cell_w[e + k] : 0.f;
+      v[k] = k < m ? sc[(size_t)d.cell_idx[e + k] * C] : c2(0.f, 0.f);
     }
+    acc += v[0] * w[0];
 #pragma unroll
-    for (int c = 0; c < MAXC; ++c)
-      if (c < nc) H[(size_t)(cbase + c) * ncell + cell] = acc[c];
+    for (int k = 1; k < 4; ++k)
+      if (k < m) acc += v[k] * w[k];
   }
+  H[i] = acc;
 }
 
 // IFFT along y of each grid column; keep the N image rows -> T[c][gx][y].
@@ -269,8 +248,8 @@ __global__ void __launch_bounds__(kRT) rad_cols_inv(RadDev d, const float2* __re
   const int ncb = min(kRC, d.G - gx0);
   for (int i = threadIdx.x; i < d.G; i += blockDim.x) tw[i] = d.tw[i];
   for (int i = threadIdx.x; i < ncb * d.G; i += blockDim.x) {
-    const int cb = i / d.G, gy = i - cb * d.G;
-    A[cb * d.ldG + gy] = H[((size_t)c * d.G + gx0 + cb) * d.G + gy];
+    const int gy = i / ncb, cb = i - gy * ncb;
+    A[cb * d.ldG + gy] = H[((size_t)gy * d.G + gx0 + cb) * d.C + c];
   }
   __syncthreads();
   const float2* X = smem_fft(A, B, ncb, d.ldG, d.plan, tw, true);
@@ -372,18 +351,18 @@ class RadialOp : public OpImpl, public SolverHooks {
   }
   SolverHooks* hooks() override { return this; }
 
-  // SolverHooks: the k-space layout is the user layout (C, Ns).
+  // SolverHooks: the compact k-space layout is the user layout (C, Ns) transposed.
   size_t compact_elems() override {
     prepare();
     return (size_t)dev_.C * dev_.Ns;
   }
   void gather(const float2* dense, float2* compact, cudaStream_t st) override {
     prepare();
-    PDT_CUDA_CHECK(cudaMemcpyAsync(compact, dense, sizeof(float2) * dev_.C * dev_.Ns, cudaMemcpyDeviceToDevice, st));
+    launch_transpose(dense, compact, 0, st);
   }
   void scatter(const float2* compact, float2* dense, cudaStream_t st) override {
     prepare();
-    PDT_CUDA_CHECK(cudaMemcpyAsync(dense, compact, sizeof(float2) * dev_.C * dev_.Ns, cudaMemcpyDeviceToDevice, st));
+    launch_transpose(compact, dense, 1, st);
   }
   int groups() override {
     prepare();
@@ -401,7 +380,7 @@ class RadialOp : public OpImpl, public SolverHooks {
   }
   void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool) override {
     prepare();
-    launch_weight(fc, st);
+    launch_weight(fc, 0, st);
     adjoint_from_weighted(svals_.as<float2>(), img, 1, st, nullptr);
   }
 
@@ -422,7 +401,7 @@ class RadialOp : public OpImpl, public SolverHooks {
   }
   void execute_adjoint(const float2* src, float2* dst, cudaStream_t st) override {
     prepare();
-    launch_weight(src, st);
+    launch_weight(src, 1, st);
     adjoint_from_weighted(svals_.as<float2>(), dst, 1, st, nullptr);
   }
   void invalidate() override { prepared_ = false; }
@@ -451,38 +430,38 @@ class RadialOp : public OpImpl, public SolverHooks {
   // mode 0: kout = A u; mode 1: k-space dual prox into r and the weighted samples svals_
   void launch_degrid(int mode, float2* kout, float2* r, const float2* fc, float sigma, float lambda,
                      cudaStream_t st) {
-    constexpr int kDegridCoils = 4;  // coils per thread; the chunks are spread over grid.y
-    const dim3 nb((dev_.Ns + kRT - 1) / kRT, (dev_.C + kDegridCoils - 1) / kDegridCoils);
-    if (dev_.kw == 3)
-      rad_degrid<kDegridCoils, 3><<<nb, kRT, 0, st>>>(dev_, mode, grid_.as<float2>(), kout, r, fc, svals_.as<float2>(),
-                                                      sigma, lambda);
-    else
-      rad_degrid<kDegridCoils, 0><<<nb, kRT, 0, st>>>(dev_, mode, grid_.as<float2>(), kout, r, fc, svals_.as<float2>(),
-                                                      sigma, lambda);
-    PDT_LAUNCH_CHECK();
+    if (!dev_.Ns) return;
+    LaunchEx lx(dim3((unsigned)(((size_t)dev_.Ns * dev_.C + kRT - 1) / kRT)), dim3(kRT), 0, st);
+    PDT_CUDA_CHECK(cudaLaunchKernelEx(&lx.cfg, dev_.kw == 3 ? rad_degrid<3> : rad_degrid<0>, dev_, mode,
+                                      (const float2*)grid_.as<float2>(), kout, r, fc, svals_.as<float2>(), sigma, lambda));
     count_launch();
   }
 
-  void launch_weight(const float2* k, cudaStream_t st) {
+  void launch_weight(const float2* k, int dense, cudaStream_t st) {
     const size_t n = (size_t)dev_.C * dev_.Ns;
-    rad_weight<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, st>>>(dev_, k, svals_.as<float2>());
+    if (!n) return;
+    rad_weight<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, st>>>(dev_, k, dense, svals_.as<float2>());
+    PDT_LAUNCH_CHECK();
+    count_launch();
+  }
+  void launch_transpose(const float2* in, float2* out, int to_dense, cudaStream_t st) {
+    const size_t n = (size_t)dev_.C * dev_.Ns;
+    if (!n) return;
+    rad_transpose<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, st>>>(dev_, in, out, to_dense);
     PDT_LAUNCH_CHECK();
     count_launch();
   }
 
   // grid_ <- FFT2 of the deapodised, zero-padded coil images.
   void forward_grid(const float2* u, cudaStream_t st, PhaseMarker* mk) {
-    if (fast_.ok()) {
-      const int R = fast_.per_block();
-      fast_.rows_fwd<<<dim3((dev_.N + R - 1) / R, dev_.C), 32 * kRadWpb, rad_fast_rows_smem(fast_), st>>>(
-          dev_, u, tbuf_.as<float2>());
-      PDT_LAUNCH_CHECK();
-      count_launch();
+    if (rows_.ok()) {
+      LaunchEx lr(dim3(dev_.N, (dev_.C + kRadCoils - 1) / kRadCoils), dim3(kRadT), rad_rows_fwd_smem(rows_, dev_.N, dev_.C),
+                  st);
+      PDT_CUDA_CHECK(cudaLaunchKernelEx(&lr.cfg, rows_.fwd, pass(), u, tbuf_.as<float2>()));
       if (mk) mk->mark("rad_rows_fwd", st);
-      fast_.cols<<<dim3((dev_.G + R - 1) / R, dev_.C), 32 * kRadWpb, rad_fast_cols_smem(fast_), st>>>(
-          dev_, tbuf_.as<float2>(), grid_.as<float2>());
-      PDT_LAUNCH_CHECK();
-      count_launch();
+      LaunchEx lc(dim3((dev_.G * dev_.C + kRadCols - 1) / kRadCols), dim3(kRadT), rad_cols_smem(rows_), st);
+      PDT_CUDA_CHECK(cudaLaunchKernelEx(&lc.cfg, cols_.fwd, pass(), (const float2*)tbuf_.as<float2>(), grid_.as<float2>()));
+      count_launch(2);
       if (mk) mk->mark("rad_cols_fwd", st);
       return;
     }
@@ -500,28 +479,17 @@ class RadialOp : public OpImpl, public SolverHooks {
 
   // out (G partial images) <- K^H applied to the already weighted samples s.
   void adjoint_from_weighted(const float2* s, float2* out, int G, cudaStream_t st, PhaseMarker* mk) {
-    const int hblk = (dev_.n_heavy + kRT / 32 - 1) / (kRT / 32);
-    const int nblk = hblk + (int)(((size_t)dev_.G * dev_.G + kRT - 1) / kRT);
-    if (dev_.C <= 4)
-      rad_grid<4><<<nblk, kRT, 0, st>>>(dev_, s, grid_.as<float2>(), hblk);
-    else if (dev_.C <= 8)
-      rad_grid<8><<<nblk, kRT, 0, st>>>(dev_, s, grid_.as<float2>(), hblk);
-    else
-      rad_grid<16><<<nblk, kRT, 0, st>>>(dev_, s, grid_.as<float2>(), hblk);
-    PDT_LAUNCH_CHECK();
+    LaunchEx lg(dim3(dev_.n_heavy + (unsigned)(((size_t)dev_.G * dev_.G * dev_.C + kRT - 1) / kRT)), dim3(kRT), 0, st);
+    PDT_CUDA_CHECK(cudaLaunchKernelEx(&lg.cfg, rad_grid, dev_, s, grid_.as<float2>()));
     count_launch();
     if (mk) mk->mark("rad_grid", st);
-    if (fast_.ok()) {
-      const int R = fast_.per_block();
-      fast_.cols_inv<<<dim3((dev_.G + R - 1) / R, dev_.C), 32 * kRadWpb, rad_fast_cols_smem(fast_), st>>>(
-          dev_, grid_.as<float2>(), tbuf_.as<float2>());
-      PDT_LAUNCH_CHECK();
-      count_launch();
+    if (rows_.ok()) {  // one image whatever G
+      LaunchEx lc(dim3((dev_.G * dev_.C + kRadCols - 1) / kRadCols), dim3(kRadT), rad_cols_smem(rows_), st);
+      PDT_CUDA_CHECK(cudaLaunchKernelEx(&lc.cfg, cols_.inv, pass(), (const float2*)grid_.as<float2>(), tbuf_.as<float2>()));
       if (mk) mk->mark("rad_cols_inv", st);
-      fast_.rows_inv<<<dim3((dev_.N + R - 1) / R, G), 32 * kRadWpb, rad_fast_rows_inv_smem(fast_, dev_.N), st>>>(
-          dev_, tbuf_.as<float2>(), out, G, (long long)dev_.N * dev_.N);
-      PDT_LAUNCH_CHECK();
-      count_launch();
+      LaunchEx lr(dim3(dev_.N), dim3(kRadT), rad_rows_inv_smem(rows_, dev_.N, dev_.C), st);
+      PDT_CUDA_CHECK(cudaLaunchKernelEx(&lr.cfg, rows_.inv, pass(), (const float2*)tbuf_.as<float2>(), out));
+      count_launch(2);
       if (mk) mk->mark("rad_rows_inv", st);
       return;
     }
@@ -605,7 +573,7 @@ class RadialOp : public OpImpl, public SolverHooks {
     for (int j = 0; j < Ns; ++j)
       for (int ty = 0; ty < kw; ++ty)
         for (int txx = 0; txx < kw; ++txx)
-          ++ptr[(size_t)wrap(g0[2 * j] + txx) * G + wrap(g0[2 * j + 1] + ty) + 1];
+          ++ptr[(size_t)wrap(g0[2 * j + 1] + ty) * G + wrap(g0[2 * j] + txx) + 1];
     for (size_t c = 0; c < ncell; ++c) ptr[c + 1] += ptr[c];
     std::vector<int> idx((size_t)ptr[ncell]), fill(ptr.begin(), ptr.end() - 1);
     std::vector<float> cw(idx.size());
@@ -615,7 +583,7 @@ class RadialOp : public OpImpl, public SolverHooks {
     for (int j = 0; j < Ns; ++j)
       for (int txx = 0; txx < kw; ++txx)
         for (int ty = 0; ty < kw; ++ty) {
-          const size_t cell = (size_t)wrap(g0[2 * j] + txx) * G + wrap(g0[2 * j + 1] + ty);
+          const size_t cell = (size_t)wrap(g0[2 * j + 1] + ty) * G + wrap(g0[2 * j] + txx);
           const int e = fill[cell]++;
           idx[e] = j;
           cw[e] = wt[((size_t)j * 2 + 0) * kw + txx] * wt[((size_t)j * 2 + 1) * kw + ty];
@@ -623,7 +591,7 @@ class RadialOp : public OpImpl, public SolverHooks {
     std::vector<float2> tw(G);
     fill_twiddles(G, tw.data());
     std::vector<float> w(dcf, dcf + Ns);
-    const size_t need = 64 * 10 + sizeof(float2) * G + sizeof(float) * (N + (size_t)Ns + wt.size() + cw.size()) +
+    const size_t need = 64 * 11 + 2 * sizeof(float2) * G + sizeof(float) * (N + (size_t)Ns + wt.size() + cw.size()) +
                         sizeof(int) * (g0.size() + ptr.size() + idx.size() + heavy.size());
     tables_.ensure(need);
     char* base = tables_.as<char>();
@@ -648,23 +616,26 @@ class RadialOp : public OpImpl, public SolverHooks {
     tbuf_.ensure(sizeof(float2) * (size_t)C * G * N);
     grid_.ensure(sizeof(float2) * (size_t)C * G * G);
     svals_.ensure(sizeof(float2) * std::max<size_t>((size_t)C * Ns, 1));
-    // lane-FFT passes where the grid length has a compiled split
-    fast_ = find_rad_kernels(G);
-    if (fast_.ok() && (rad_fast_rows_inv_smem(fast_, N) > (size_t)g_rad_smem ||
-                       rad_fast_cols_smem(fast_) > (size_t)g_rad_smem))
-      fast_ = RadFastKernels();
-    if (fast_.ok()) {
-      for (const void* fn : {(const void*)fast_.rows_fwd, (const void*)fast_.cols, (const void*)fast_.cols_inv,
-                             (const void*)fast_.rows_inv})
+    // register transforms where the grid length has a compiled split
+    rows_ = find_rad_rows(G);
+    cols_ = find_rad_cols(G);
+    if (rows_.ok() && std::max({rad_rows_inv_smem(rows_, N, C), rad_rows_fwd_smem(rows_, N, C), rad_cols_smem(rows_)}) >
+                          (size_t)g_rad_smem)
+      rows_ = RadRowKernels();
+    if (rows_.ok()) {
+      std::vector<float2> tw2(G);
+      for (int t = 0; t < rows_.Q; ++t)
+        for (int k1 = 0; k1 < rows_.P; ++k1) tw2[t * rows_.P + k1] = tw[t * k1];  // t k1 < G
+      tw2_ = reinterpret_cast<const float2*>(put(tw2.data(), sizeof(float2) * G));
+      for (const void* fn : {(const void*)rows_.fwd, (const void*)rows_.inv, (const void*)cols_.fwd, (const void*)cols_.inv})
         PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g_rad_smem));
     }
-    const int rows_per_block = fast_.ok() ? fast_.per_block() : kRR;
-    const int row_blocks = (N + rows_per_block - 1) / rows_per_block;
-    G_ = std::max(1, std::min(C, (2 * g_rad_sms + row_blocks - 1) / row_blocks));
+    const int row_blocks = (N + kRR - 1) / kRR;
+    G_ = rows_.ok() ? 1 : std::max(1, std::min(C, (2 * g_rad_sms + row_blocks - 1) / row_blocks));
     if (const char* env = std::getenv("PDT_RADIAL_GROUPS")) {  // coil groups of the adjoint row pass, pinned
       const int g = std::atoi(env);
       if (g < 1 || g > C) throw Error(PDT_ERR_INVALID_ARGUMENT, "PDT_RADIAL_GROUPS must be 1 .. coils");
-      G_ = g;
+      if (!rows_.ok()) G_ = g;
     }
     dev_ = d;
     prepared_ = true;
@@ -674,7 +645,10 @@ class RadialOp : public OpImpl, public SolverHooks {
   int64_t sector_width_ = 0, kernel_width_ = 0, img_dim_ = 0;
   bool prepared_ = false;
   RadDev dev_{};
-  RadFastKernels fast_;
+  RadRowKernels rows_;
+  RadColKernels cols_;
+  const float2* tw2_ = nullptr;
+  RadPass pass() const { return RadPass{dev_.N, dev_.G, dev_.C, dev_.off, dev_.scale, dev_.sens, dev_.deap, tw2_}; }
   int G_ = 1;
   DevBuf tables_, tbuf_, grid_, svals_;
 };
