@@ -279,9 +279,6 @@ class OptImpl {
     graph_.reset();
     if (own_) cudaStreamDestroy(own_);
     if (cap_) cudaStreamDestroy(cap_);
-    if (aux_) cudaStreamDestroy(aux_);
-    if (ev_fork_) cudaEventDestroy(ev_fork_);
-    if (ev_join_) cudaEventDestroy(ev_join_);
   }
 
   bool with_op() const { return kind_ == PDT_OPT_TV_OP || kind_ == PDT_OPT_TGV_OP || kind_ == PDT_OPT_TGV_MRI; }
@@ -619,12 +616,6 @@ class OptImpl {
     if (!cap_) PDT_CUDA_CHECK(cudaStreamCreateWithFlags(&cap_, cudaStreamNonBlocking));
     return cap_;
   }
-  // side stream and fork/join events of the concurrent dual update
-  void ensure_aux() {
-    if (!aux_) PDT_CUDA_CHECK(cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking));
-    if (!ev_fork_) PDT_CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
-    if (!ev_join_) PDT_CUDA_CHECK(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
-  }
 
  private:
   static void copy_in(void* dst, const void* src, size_t bytes, bool is_device, cudaStream_t st) {
@@ -777,7 +768,8 @@ class OptImpl {
     // alpha table for every iteration (tgvmrioptimizer.cu:144-155 in real_type)
     const unsigned K = params_.max_iter;
     const int n = (int)K + 1;
-    const int ld = gram ? 4 : 2;  // with line_gram(): {alpha0, alpha1, c, d}, c and d as in pdt_gram.h
+    const bool fused = !gram && hk->can_fuse_dual(W_, H_);
+    const int ld = fused ? 2 : 4;  // {alpha0, alpha1} or {alpha0, alpha1, c, d}, c and d as in pdt_gram.h
     std::vector<float> tab(ld * (size_t)n);
     double gc = 0, gd = 1;
     const float gk = sigma / (1.0f + sigma * lambda);
@@ -786,7 +778,7 @@ class OptImpl {
       if (kind_ == PDT_OPT_TGV_MRI) alpha_at(k, a0, a1);
       tab[ld * k] = a0;
       tab[ld * k + 1] = a1;
-      if (gram) {
+      if (!fused) {
         gc += (double)gk * (1.0 - (double)lambda * gc);
         gd -= (double)gk * (double)lambda * gd;
         tab[ld * k + 2] = (float)gc;
@@ -817,7 +809,7 @@ class OptImpl {
       alpha_host_ = tab;
     }
     PDT_CUDA_CHECK(cudaMemsetAsync(iter, 0, sizeof(int), st));  // the primal kernel advances it
-    if (gram) PDT_CUDA_CHECK(cudaMemsetAsync(iter + 4, 0, 2 * sizeof(int), st));  // or the one-launch iteration these
+    if (!fused) PDT_CUDA_CHECK(cudaMemsetAsync(iter + 4, 0, 2 * sizeof(int), st));  // the image kernel's counters
     const bool is_tgv = kind_ != PDT_OPT_TV_OP;
     const int p0 = parity_;
     const float* atab = reinterpret_cast<const float*>(alpha_.as<char>() + kAlphaHeader);
@@ -826,36 +818,16 @@ class OptImpl {
     pl.n = n;
     pl.p0 = p0;
     pl.verbose = verbose;
-    if (gram) {
-      plan_gram(pl, *gram, hk, r_zero, tau, sigma, lambda, gk, (float)gc, (float)gd, st);
+    if (!fused) {
+      plan_image(pl, gram, hk, G, r_zero, tau, sigma, lambda, gk, (float)gc, (float)gd, st);
       return pl;
     }
-    ensure_aux();
-    cudaStream_t aux = aux_;
-    cudaEvent_t ev_fork = ev_fork_, ev_join = ev_join_;
-    // one iteration: the dual update runs inside the operator's round where the operator has idle
-    // blocks for it (profiling then times it as part of that launch), else on `aux`, forked from and
-    // joined back into `s`, concurrently with the round (profiling runs it in line so that every phase
-    // has its own interval)
-    const bool fused = hk->can_fuse_dual(W_, H_);
+    // the dual update in the operator's round, which has idle blocks for it
     pl.body = [=](int par, cudaStream_t s) {
       const int in = p0 ^ par, out = in ^ 1;
       const float2* ubar = static_cast<const float2*>(field(F_UB, in));
-      if (fused) {
-        const DualStep ds{ptrs(in), ptrs(out), sigma, atab, iter, W_, H_, is_tgv ? 1 : 0};
-        hk->round(ubar, r_.as<float2>(), fc_.as<float2>(), sigma, lambda, khr, nullptr, s, prof_, &ds);
-      } else if (prof_) {
-        launch_mri_dual(is_tgv, W_, H_, ptrs(in), ptrs(out), sigma, atab, iter, s);
-        prof_->mark(is_tgv ? "mri_dual_tgv" : "mri_dual_tv", s);
-        hk->round(ubar, r_.as<float2>(), fc_.as<float2>(), sigma, lambda, khr, nullptr, s, prof_);
-      } else {
-        PDT_CUDA_CHECK(cudaEventRecord(ev_fork, s));
-        PDT_CUDA_CHECK(cudaStreamWaitEvent(aux, ev_fork, 0));
-        launch_mri_dual(is_tgv, W_, H_, ptrs(in), ptrs(out), sigma, atab, iter, aux);
-        PDT_CUDA_CHECK(cudaEventRecord(ev_join, aux));
-        hk->round(ubar, r_.as<float2>(), fc_.as<float2>(), sigma, lambda, khr, nullptr, s, nullptr);
-        PDT_CUDA_CHECK(cudaStreamWaitEvent(s, ev_join, 0));
-      }
+      const DualStep ds{ptrs(in), ptrs(out), sigma, atab, iter, W_, H_, is_tgv ? 1 : 0};
+      hk->round(ubar, r_.as<float2>(), fc_.as<float2>(), sigma, lambda, khr, nullptr, s, prof_, &ds);
       launch_mri_primal(is_tgv, W_, H_, ptrs(out), khr, G, gstride, tau, iter, s);
       if (prof_) prof_->mark(is_tgv ? "mri_primal_tgv" : "mri_primal_tv", s);
     };
@@ -867,42 +839,46 @@ class OptImpl {
     return pl;
   }
 
-  // The iterations with a line mask's row operator (pdt_gram.h): b = K^H f and z0 = K^H r_0, the first dual
-  // update and U; two launches an iteration; then the k-space dual from U. u, v, U alternate between two copies
-  // with the iteration (the free halves of the slab), p and q with the state's parity. An error of b acts like
-  // one of the data in every iteration, so its rows are transformed in FP32 (with the tensor-core rows u was
-  // 1.5e-6 off after 1001 iterations instead of 5e-7).
-  void plan_gram(Plan& pl, const GramRows& rows, SolverHooks* hk, bool r_zero, float tau, float sigma, float lambda,
-                 float k, float c, float d, cudaStream_t st) {
+  // Iterations of an operator part and one image kernel (launch_gram_image): the primal update, then the next
+  // iteration's dual update, whose first one runs here. The operator part is the round with the k-space dual, or for a
+  // line mask the row operator (pdt_gram.h): then b = K^H f and z0 = K^H r_0 are formed here and the k-space dual
+  // follows from U after the iterations. u, v, U alternate between two copies with the iteration (the free halves of
+  // the slab), p and q with the state's parity. An error of b acts like one of the data in every iteration, so its
+  // rows are transformed in FP32 (with the tensor-core rows u was 1.5e-6 off after 1001 iterations instead of 4e-7).
+  void plan_image(Plan& pl, const GramRows* gram, SolverHooks* hk, int G, bool r_zero, float tau, float sigma,
+                  float lambda, float k, float c, float d, cudaStream_t st) {
     const size_t N = (size_t)W_ * H_, plane = plane_bytes();
-    const size_t bytes = (6 + (size_t)rows.groups) * plane;
-    if (gram_.bytes != bytes) {
-      gram_.ensure(bytes);
-      ++version_;
-    }
-    float2* U = gram_.as<float2>();  // two copies of {U, compensation}, b, z0, partial sums
-    float2* b = U + 4 * N;
-    float2* z0 = b + N;
-    float2* part = z0 + N;
-    hk->adjoint_compact(fc_.as<float2>(), b, st, true);
-    if (!r_zero) hk->adjoint_compact(r_.as<float2>(), z0, st, true);
-    const int p0 = parity_, n = pl.n;
+    const bool row_op = gram != nullptr;
+    const GramRows rows = row_op ? *gram : GramRows();
+    const int p0 = parity_, n = pl.n, groups = row_op ? rows.groups : G;
     const bool is_tgv = kind_ != PDT_OPT_TV_OP;
     int* header = alpha_.as<int>();
     const float4* table = reinterpret_cast<const float4*>(alpha_.as<char>() + kAlphaHeader);
-    {
-      // the first dual update reads {alpha0, alpha1} of row 0 whatever the row length
-      launch_mri_dual(is_tgv, W_, H_, ptrs(p0), ptrs(p0 ^ 1), sigma, reinterpret_cast<const float*>(table), header, st);
+    float2 *U = nullptr, *b = nullptr, *z0 = nullptr, *part = khr_.as<float2>();
+    if (row_op) {  // two copies of {U, compensation}, b, z0, partial sums
+      const size_t bytes = (6 + (size_t)groups) * plane;
+      if (gram_.bytes != bytes) {
+        gram_.ensure(bytes);
+        ++version_;
+      }
+      U = gram_.as<float2>();
+      b = U + 4 * N;
+      z0 = b + N;
+      part = z0 + N;
+      hk->adjoint_compact(fc_.as<float2>(), b, st, true);
+      if (!r_zero) hk->adjoint_compact(r_.as<float2>(), z0, st, true);
       launch_gram_start(W_, H_, static_cast<const float2*>(field(F_UB, p0)), k, U, st);
     }
-    if (prof_) prof_->mark("mri_gram_setup", st);
+    // reads {alpha0, alpha1} of row 0 whatever the row length
+    launch_mri_dual(is_tgv, W_, H_, ptrs(p0), ptrs(p0 ^ 1), sigma, reinterpret_cast<const float*>(table), header, st);
+    if (prof_) prof_->mark("mri_setup", st);
     pl.body = [=](int par, cudaStream_t s) {
       GramImage g{};
       g.W = W_;
       g.H = H_;
       g.src = ptrs(p0 ^ par ^ 1);  // this iteration's p, q
       g.dst = ptrs(p0 ^ par);      // the next one's
-      g.dst.ub = g.src.ub;         // u-bar and v-bar of the last iteration join its p, q
+      g.dst.ub = g.src.ub;         // u-bar and (the last iteration's) v-bar join its p, q
       g.dst.vbx = g.src.vbx;
       g.dst.vby = g.src.vby;
       auto primal = [&](ImgPtrs& q, int set) {
@@ -912,12 +888,14 @@ class OptImpl {
       };
       primal(g.src, par);
       primal(g.dst, par ^ 1);
-      g.U = U + 2 * N * par;
-      g.Unext = U + 2 * N * (par ^ 1);
+      if (row_op) {
+        g.U = U + 2 * N * par;
+        g.Unext = U + 2 * N * (par ^ 1);
+        g.b = b;
+        g.z0 = r_zero ? nullptr : z0;
+      }
       g.part = part;
-      g.groups = rows.groups;
-      g.b = b;
-      g.z0 = r_zero ? nullptr : z0;
+      g.groups = groups;
       g.table = table;
       g.header = header;
       g.par = par;
@@ -925,22 +903,28 @@ class OptImpl {
       g.sigma = sigma;
       g.lambda = lambda;
       g.k = k;
-      launch_gram_rows(rows, g.U, part, s);
-      if (prof_) prof_->mark("mri_gram_rows", s);
-      launch_gram_image(is_tgv, g, s);
-      if (prof_) prof_->mark(is_tgv ? "mri_gram_image_tgv" : "mri_gram_image_tv", s);
+      if (row_op) {
+        launch_gram_rows(rows, g.U, part, s);
+        if (prof_) prof_->mark("mri_gram_rows", s);
+      } else {
+        hk->round(static_cast<const float2*>(field(F_UB, p0 ^ par)), r_.as<float2>(), fc_.as<float2>(), sigma, lambda,
+                  part, nullptr, s, prof_);
+      }
+      launch_gram_image(is_tgv, row_op, g, s);
+      if (prof_) prof_->mark(is_tgv ? "mri_image_tgv" : "mri_image_tv", s);
     };
     pl.post = [=](cudaStream_t s) {
       if (n & 1)  // the results lie in the second copies
         for (int f : {(int)F_U, (int)F_VX, (int)F_VY})
           if (f == F_U || is_tgv)
             PDT_CUDA_CHECK(cudaMemcpyAsync(raw_field(f, 0), raw_field(f, 1), plane, cudaMemcpyDeviceToDevice, s));
-      hk->dual_from_image(U + 2 * N * ((n - 1) & 1), r_.as<float2>(), fc_.as<float2>(), c, d, s);
-      if (prof_) prof_->mark("mri_gram_dual", s);
+      if (row_op) hk->dual_from_image(U + 2 * N * ((n - 1) & 1), r_.as<float2>(), fc_.as<float2>(), c, d, s);
+      if (prof_) prof_->mark("mri_finish", s);
     };
-    pl.key = graph_key({(uintptr_t)img_.p, (uintptr_t)gram_.p, (uintptr_t)alpha_.p, (uintptr_t)alpha_.bytes,
-                        (uintptr_t)op_.get(), (uintptr_t)op_->generation(), (uintptr_t)W_, (uintptr_t)H_, (uintptr_t)p0,
-                        (uintptr_t)is_tgv, (uintptr_t)r_zero, fbits(lambda), fbits(tau), fbits(sigma),
+    pl.key = graph_key({(uintptr_t)img_.p, (uintptr_t)gram_.p, (uintptr_t)khr_.p, (uintptr_t)r_.p, (uintptr_t)fc_.p,
+                        (uintptr_t)alpha_.p, (uintptr_t)alpha_.bytes, (uintptr_t)op_.get(), (uintptr_t)op_->generation(),
+                        (uintptr_t)W_, (uintptr_t)H_, (uintptr_t)groups, (uintptr_t)p0, (uintptr_t)is_tgv,
+                        (uintptr_t)r_zero, (uintptr_t)row_op, fbits(lambda), fbits(tau), fbits(sigma),
                         (uintptr_t)version_, (uintptr_t)1});
   }
 
@@ -1014,8 +998,7 @@ class OptImpl {
   IterGraph graph_;
   PhaseMarker* prof_ = nullptr;
   bool profiling_ = false;
-  cudaStream_t own_ = nullptr, cap_ = nullptr, aux_ = nullptr;
-  cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
+  cudaStream_t own_ = nullptr, cap_ = nullptr;
 };
 
 

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
 // ------------------------------------------------------------------------------------------------
 constexpr int GX = 32, GY = 8, GT = 320;  // (GX + 1) (GY + 1) = 297 primal pixels, one a thread
 
-template <bool TGV>
+template <bool TGV, bool ROWS>
 __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   __shared__ float2 s_px[GY + 2][GX + 2], s_py[GY + 2][GX + 2];  // [x0 - 1, x0 + GX] x [y0 - 1, y0 + GY]
   __shared__ float2 s_qxx[TGV ? GY + 2 : 1][GX + 2], s_qyy[TGV ? GY + 2 : 1][GX + 2], s_qxy[TGV ? GY + 2 : 1][GX + 2];
@@ -191,13 +191,15 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   float2 ou = c2(0.f, 0.f), kf = ou, ovx = ou, ovy = ou, Uo = ou, Ue = ou;
   if (in) {
     ou = ld(s.src.u, idx);
-    kf = row.z * __ldcg(s.b + idx);
-    if (s.z0) kf = kf - row.w * __ldcg(s.z0 + idx);
+    if constexpr (ROWS) {
+      kf = row.z * __ldcg(s.b + idx);
+      if (s.z0) kf = kf - row.w * __ldcg(s.z0 + idx);
+    }
     if constexpr (TGV) {
       ovx = ld(s.src.vx, idx);
       ovy = ld(s.src.vy, idx);
     }
-    if (own) {
+    if (ROWS && own) {
       Uo = __ldcg(s.U + idx);
       Ue = __ldcg(s.U + (size_t)W * H + idx);
     }
@@ -252,7 +254,8 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   if (in) {
     float2 kh = s.part[idx];
     for (int g = 1; g < s.groups; ++g) kh += s.part[idx + (size_t)g * W * H];
-    const float2 un = ou + s.tau * (dp - (kh - kf));
+    if constexpr (ROWS) kh = kh - kf;
+    const float2 un = ou + s.tau * (dp - kh);
     s_ub[ly][lx] = 2.0f * un - ou;
     finite = finite && isfinite(un.x) && isfinite(un.y);
     if (own) static_cast<float2*>(s.dst.u)[idx] = un;
@@ -261,10 +264,8 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   __syncthreads();
   if (!own) return;
   const float2 c = s_ub[ly][lx];
-  if (it >= last) {
-    static_cast<float2*>(s.dst.ub)[idx] = c;
-    return;
-  }
+  if (!ROWS || it >= last) static_cast<float2*>(s.dst.ub)[idx] = c;
+  if (it >= last) return;
   // the next iteration's p (tgv_kernels.cuh:260-292)
   float2 gx = s_ub[ly][xp] - c, gy = s_ub[yp][lx] - c;
   if constexpr (TGV) {
@@ -275,6 +276,7 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   const float sp = dual_proj_scale(sqrtf(abs2(a) + abs2(b)), TGV ? next.y : 1.0f);
   static_cast<float2*>(s.dst.px)[idx] = a * sp;
   static_cast<float2*>(s.dst.py)[idx] = b * sp;
+  if constexpr (!ROWS) return;
   // U + its compensation
   auto step = [&](float u, float e, float ub, float& nu, float& ne) {
     const float inc = __fadd_rn(e, s.k * ((ub - s.lambda * u) - s.lambda * e));
@@ -402,9 +404,11 @@ void launch_gram_rows(const GramRows& g, const float2* U, float2* part, cudaStre
   throw Error(PDT_ERR_STATE, "no row kernel for transform length " + std::to_string(g.len.n));
 }
 
-void launch_gram_image(bool tgv, const GramImage& s, cudaStream_t st) {
+void launch_gram_image(bool tgv, bool rows, const GramImage& s, cudaStream_t st) {
   LaunchEx lx(dim3((s.W + GX - 1) / GX, (s.H + GY - 1) / GY), dim3(GT), 0, st);
-  PDT_CUDA_CHECK(cudaLaunchKernelEx(&lx.cfg, tgv ? gram_image_kernel<true> : gram_image_kernel<false>, s));
+  auto fn = tgv ? (rows ? gram_image_kernel<true, true> : gram_image_kernel<true, false>)
+                : (rows ? gram_image_kernel<false, true> : gram_image_kernel<false, false>);
+  PDT_CUDA_CHECK(cudaLaunchKernelEx(&lx.cfg, fn, s));
   count_launch();
 }
 

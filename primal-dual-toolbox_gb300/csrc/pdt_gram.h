@@ -54,7 +54,7 @@ void gram_tables(int W, const GramLength& len, const std::vector<float>& m2, std
 struct GramImage {
   int W, H;
   ImgPtrs src;           // u, v and the p, q of this iteration
-  ImgPtrs dst;           // new u, v; ubar, vbar (last iteration only); p, q of the next iteration
+  ImgPtrs dst;           // new u, v; ubar, vbar (last iteration only, see launch_gram_image); p, q of the next
   const float2* U;       // this iteration's U, then its compensation (W x H each)
   float2* Unext;
   const float2* part;    // `groups` partial sums of K^H K U, W x H each
@@ -70,8 +70,10 @@ struct GramImage {
 // part[g] <- sum of conj(s_c) . G (s_c . U) over the coils of group g.
 void launch_gram_rows(const GramRows& g, const float2* U, float2* part, cudaStream_t st);
 // u, v <- the primal update from part; then, unless this is the table's last iteration, p, q and U of the
-// next one (the last iteration stores ubar and vbar instead). Raises header[2] on a non-finite u or v.
-void launch_gram_image(bool tgv, const GramImage& s, cudaStream_t st);
+// next one (the last iteration stores ubar and vbar instead). Raises header[2] on a non-finite u or v. Without
+// `rows`, part holds K^H r itself: U, b, z0 are not used and every iteration stores ubar, which the next operator
+// round reads.
+void launch_gram_image(bool tgv, bool rows, const GramImage& s, cudaStream_t st);
 // U <- k ubar, compensation 0: the first iteration's U, from U_0 = 0.
 void launch_gram_start(int W, int H, const float2* ubar, float k, float2* U, cudaStream_t st);
 

@@ -110,17 +110,37 @@ __global__ void __launch_bounds__(kRT) rad_cols(RadDev d, const float2* __restri
   }
 }
 
-// Degridding, a thread per (sample, coil), coils fastest. mode 0: kout[c][j] = A u (the user's layout). mode 1
+// V consecutive coil values (V = 2: one 16-byte access; C even, so runs start on 16 bytes).
+template <int V>
+__device__ __forceinline__ void ld_run(float2 (&v)[V], const float2* p) {
+  if constexpr (V == 2) {
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = c2(t.x, t.y);
+    v[1] = c2(t.z, t.w);
+  } else {
+    v[0] = *p;
+  }
+}
+template <int V>
+__device__ __forceinline__ void st_run(float2* p, const float2 (&v)[V]) {
+  if constexpr (V == 2)
+    *reinterpret_cast<float4*>(p) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+  else
+    *p = v[0];
+}
+
+// Degridding, a thread per (sample, V coils), coils fastest. mode 0: kout[c][j] = A u (the user's layout). mode 1
 // (solver): r <- (r + sigma (A u - f)) / (1 + sigma lambda), s[j][c] = w_j r (the weighted values the adjoint
 // grids). KW > 0 fixes the kernel width at compile time so that the taps unroll (KW = 0: d.kw at run time). Bound by L2:
 // KW^2 runs of C values a sample (12 coils, 32768 samples: 28 MB).
-template <int KW>
+template <int KW, int V>
 __global__ void __launch_bounds__(kRT) rad_degrid(RadDev d, int mode, const float2* __restrict__ F,
                                                   float2* __restrict__ kout, float2* __restrict__ r,
                                                   const float2* __restrict__ f, float2* __restrict__ s,
                                                   float sigma, float lambda) {
-  const unsigned i = blockIdx.x * kRT + threadIdx.x;
-  const unsigned j = i / (unsigned)d.C, c = i - j * (unsigned)d.C;
+  const unsigned nv = (unsigned)d.C / V, q = blockIdx.x * kRT + threadIdx.x;
+  const unsigned j = q / nv, c = V * (q - j * nv);
+  const size_t i = (size_t)j * d.C + c;
   const bool ok = j < (unsigned)d.Ns;
   static_assert(KW >= 0 && KW <= kMaxKw, "kernel width");
   const int kw = KW > 0 ? KW : d.kw;
@@ -140,22 +160,42 @@ __global__ void __launch_bounds__(kRT) rad_degrid(RadDev d, int mode, const floa
   pdl_wait();  // F comes from the previous kernel
   pdl_trigger();
   if (!ok) return;
-  const float2 ro = mode ? r[i] : c2(0.f, 0.f), fo = mode ? f[i] : c2(0.f, 0.f);
-  float2 a = c2(0.f, 0.f);
+  float2 ro[V], fo[V], a[V];
+  if (mode) {
+    ld_run<V>(ro, r + i);
+    ld_run<V>(fo, f + i);
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) a[v] = c2(0.f, 0.f);
 #pragma unroll
   for (int tx = 0; tx < kw; ++tx) {
-    float2 col = c2(0.f, 0.f);
+    float2 col[V];
 #pragma unroll
-    for (int ty = 0; ty < kw; ++ty) col += F[(size_t)(gys[ty] + gxs[tx]) * d.C + c] * wy[ty];
-    a += col * wx[tx];
+    for (int v = 0; v < V; ++v) col[v] = c2(0.f, 0.f);
+#pragma unroll
+    for (int ty = 0; ty < kw; ++ty) {
+      float2 t[V];
+      ld_run<V>(t, F + (size_t)(gys[ty] + gxs[tx]) * d.C + c);
+#pragma unroll
+      for (int v = 0; v < V; ++v) col[v] += t[v] * wy[ty];
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) a[v] += col[v] * wx[tx];
   }
-  const float2 av = a * wj;
-  if (mode == 0) {
-    kout[(size_t)c * d.Ns + j] = av;
-  } else {
-    const float2 rn = (ro + sigma * (av - fo)) / (1.0f + sigma * lambda);
-    r[i] = rn;
-    s[i] = rn * wj;
+  float2 rn[V], sn[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const float2 av = a[v] * wj;
+    if (mode == 0) {
+      kout[(size_t)(c + v) * d.Ns + j] = av;
+    } else {
+      rn[v] = (ro[v] + sigma * (av - fo[v])) / (1.0f + sigma * lambda);
+      sn[v] = rn[v] * wj;
+    }
+  }
+  if (mode) {
+    st_run<V>(r + i, rn);
+    st_run<V>(s + i, sn);
   }
 }
 
@@ -186,6 +226,7 @@ __global__ void rad_transpose(RadDev d, const float2* __restrict__ in, float2* _
 // every slots-th entry and the slots added in order; the others give each (cell, coil) a thread that walks the
 // cell's list in order, four entries at a time so that many loads are in flight. A warp's loads of s are runs of C
 // values (a thread per cell and all coils, as before, touched 32 runs a load: 20 us instead of 6 for 12 coils on 384^2).
+template <int V>
 __global__ void __launch_bounds__(kRT) rad_grid(RadDev d, const float2* __restrict__ s, float2* __restrict__ H) {
   const int C = d.C;
   if ((int)blockIdx.x < d.n_heavy) {
@@ -212,30 +253,35 @@ __global__ void __launch_bounds__(kRT) rad_grid(RadDev d, const float2* __restri
     }
     return;
   }
+  const unsigned nv = (unsigned)C / V;
   const size_t i = (blockIdx.x - d.n_heavy) * (size_t)kRT + threadIdx.x;
-  const unsigned cell = (unsigned)(i / (unsigned)C);
+  const unsigned cell = (unsigned)(i / nv), c = V * (unsigned)(i - (size_t)cell * nv);
   const bool ok = cell < (unsigned)(d.G * d.G);
   const int beg = ok ? d.cell_ptr[cell] : 0, end = ok ? d.cell_ptr[cell + 1] : 0;
-  const float2* sc = s + (i - (size_t)cell * C);
   pdl_wait();
   pdl_trigger();
   if (!ok || end - beg > kHeavy) return;  // a block of its own grids it
-  float2 acc = c2(0.f, 0.f);
+  float2 acc[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) acc[v] = c2(0.f, 0.f);
   for (int e = beg; e < end; e += 4) {
     const int m = end - e;  // entries e .. e + min(m, 4) - 1 are this cell's
-    float2 v[4];
+    float2 t[4][V];
     float w[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      w[k] = k < m ? d.cell_w[e + k] : 0.f;
-      v[k] = k < m ? sc[(size_t)d.cell_idx[e + k] * C] : c2(0.f, 0.f);
-    }
-    acc += v[0] * w[0];
+    for (int k = 0; k < 4; ++k)
+      if (k < m) {
+        w[k] = d.cell_w[e + k];
+        ld_run<V>(t[k], s + (size_t)d.cell_idx[e + k] * C + c);
+      }
 #pragma unroll
-    for (int k = 1; k < 4; ++k)
-      if (k < m) acc += v[k] * w[k];
+    for (int k = 0; k < 4; ++k)
+      if (k < m) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] += t[k][v] * w[k];
+      }
   }
-  H[i] = acc;
+  st_run<V>(H + (size_t)cell * C + c, acc);
 }
 
 // IFFT along y of each grid column; keep the N image rows -> T[c][gx][y].
@@ -431,8 +477,14 @@ class RadialOp : public OpImpl, public SolverHooks {
   void launch_degrid(int mode, float2* kout, float2* r, const float2* fc, float sigma, float lambda,
                      cudaStream_t st) {
     if (!dev_.Ns) return;
-    LaunchEx lx(dim3((unsigned)(((size_t)dev_.Ns * dev_.C + kRT - 1) / kRT)), dim3(kRT), 0, st);
-    PDT_CUDA_CHECK(cudaLaunchKernelEx(&lx.cfg, dev_.kw == 3 ? rad_degrid<3> : rad_degrid<0>, dev_, mode,
+    const int V = dev_.C % 2 ? 1 : 2;
+    LaunchEx lx(dim3((unsigned)(((size_t)dev_.Ns * dev_.C / V + kRT - 1) / kRT)), dim3(kRT), 0, st);
+    auto pick = [&](auto two, auto one) { return V == 2 ? two : one; };
+    auto fn = dev_.kw == 3   ? pick(rad_degrid<3, 2>, rad_degrid<3, 1>)
+              : dev_.kw == 4 ? pick(rad_degrid<4, 2>, rad_degrid<4, 1>)
+              : dev_.kw == 5 ? pick(rad_degrid<5, 2>, rad_degrid<5, 1>)
+                             : pick(rad_degrid<0, 2>, rad_degrid<0, 1>);
+    PDT_CUDA_CHECK(cudaLaunchKernelEx(&lx.cfg, fn, dev_, mode,
                                       (const float2*)grid_.as<float2>(), kout, r, fc, svals_.as<float2>(), sigma, lambda));
     count_launch();
   }
@@ -479,8 +531,9 @@ class RadialOp : public OpImpl, public SolverHooks {
 
   // out (G partial images) <- K^H applied to the already weighted samples s.
   void adjoint_from_weighted(const float2* s, float2* out, int G, cudaStream_t st, PhaseMarker* mk) {
-    LaunchEx lg(dim3(dev_.n_heavy + (unsigned)(((size_t)dev_.G * dev_.G * dev_.C + kRT - 1) / kRT)), dim3(kRT), 0, st);
-    PDT_CUDA_CHECK(cudaLaunchKernelEx(&lg.cfg, rad_grid, dev_, s, grid_.as<float2>()));
+    const int V = dev_.C % 2 ? 1 : 2;
+    LaunchEx lg(dim3(dev_.n_heavy + (unsigned)(((size_t)dev_.G * dev_.G * dev_.C / V + kRT - 1) / kRT)), dim3(kRT), 0, st);
+    PDT_CUDA_CHECK(cudaLaunchKernelEx(&lg.cfg, V == 2 ? rad_grid<2> : rad_grid<1>, dev_, s, grid_.as<float2>()));
     count_launch();
     if (mk) mk->mark("rad_grid", st);
     if (rows_.ok()) {  // one image whatever G
