@@ -47,11 +47,18 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// The pair of BF16 values g where the pair z is positive, else zero.
+__device__ __forceinline__ uint32_t relu_mask(uint32_t g, uint32_t z) {
+  const __nv_bfloat162 zz = *reinterpret_cast<const __nv_bfloat162*>(&z);
+  return (__bfloat162float(zz.x) > 0.f ? g & 0xFFFFu : 0u) | (__bfloat162float(zz.y) > 0.f ? g & 0xFFFF0000u : 0u);
+}
+
 enum Epi {
   EPI_RELU_RES = 2,  // zsave = z, out = in + relu(z)   (CIN == COUT)
   EPI_F32 = 3,       // out32 = z (FP32)
-  EPI_ACC = 4,       // acc32 += bf16(z)  (a residual stream's FP32 gradient; the BF16 rounding of a stored z)
-  EPI_F32_BF16 = 5   // out32 = bf16(z), stored as FP32 (starts a residual stream's gradient)
+  EPI_ACC = 4,       // acc32 += bf16(z)  (a residual stream's FP32 gradient; the BF16 rounding of a stored z), and
+                     // out = bf16(acc32) where zsave (read) > 0, else 0: the gradient at the layer below
+  EPI_F32_BF16 = 5   // out32 = bf16(z), stored as FP32 (starts a residual stream's gradient), and out likewise
 };
 
 // 32 -> 32 channel 3 x 3 convolution on the fifth-generation tensor cores (tcgen05 kind::f16, BF16
@@ -173,9 +180,13 @@ __global__ void __launch_bounds__(kConvTcThreads, 4) conv3x3_tc(const bf16* __re
     const int m = 32 * q + lane, gy = y0 + (m >> 3), gx = x0 + (m & 7);  // row m = pixel (m % 8, m / 8)
     const bool inside = gy < H && gx < W;
     const size_t pix = ((size_t)b * H + gy) * W + gx;
-    float4 acc_in[4];  // the accumulated gradient, loaded while the MMAs run
+    float4 acc_in[4];  // the accumulated gradient and the layer below's pre-activation, loaded while the MMAs run
+    uint4 zin[2];
     if constexpr (EPI == EPI_ACC) {
       if (inside) {
+        const uint4* zp = reinterpret_cast<const uint4*>(zsave + pix * CH + 16 * h);
+        zin[0] = zp[0];
+        zin[1] = zp[1];
         const float4* ap = reinterpret_cast<const float4*>(acc32 + pix * CH + 16 * h);
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) acc_in[q4] = ap[q4];
@@ -232,7 +243,15 @@ __global__ void __launch_bounds__(kConvTcThreads, 4) conv3x3_tc(const bf16* __re
           a.z += __bfloat162float(hi.x);
           a.w += __bfloat162float(hi.y);
           ap[q4] = a;
+          // ReLU's derivative on the rounded gradient (z > 0: positive, not zero, as BF16 bits)
+          const uint32_t z01 = q4 == 0 ? zin[0].x : q4 == 1 ? zin[0].z : q4 == 2 ? zin[1].x : zin[1].z;
+          const uint32_t z23 = q4 == 0 ? zin[0].y : q4 == 1 ? zin[0].w : q4 == 2 ? zin[1].y : zin[1].w;
+          o[2 * q4] = relu_mask(pack_bf16(a.x, a.y), z01);
+          o[2 * q4 + 1] = relu_mask(pack_bf16(a.z, a.w), z23);
         }
+        uint4* gp = reinterpret_cast<uint4*>(out + pix * CH + 16 * h);
+        gp[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        gp[1] = make_uint4(o[4], o[5], o[6], o[7]);
       } else {
         uint4* op = reinterpret_cast<uint4*>(out + pix * CH + 16 * h);
         op[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -262,7 +281,8 @@ __global__ void __launch_bounds__(kConvTcThreads, 4) conv3x3_tc(const bf16* __re
 template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(32 * TH) conv3x3_mma(const bf16* __restrict__ in, const bf16* __restrict__ w,
                                                        const float* __restrict__ bias, int H, int W,
-                                                       float* __restrict__ out32) {
+                                                       float* __restrict__ out32, const bf16* __restrict__ z,
+                                                       bf16* __restrict__ out) {
   static_assert(CIN % 16 == 0 && COUT % 8 == 0, "channel counts");
   static_assert(EPI == EPI_F32 || EPI == EPI_F32_BF16, "epilogues of the 32 -> 8 layer and the first data gradient");
   constexpr int PS = CIN + 4;       // smem pixel stride (bf16): spreads the fragment loads over all banks
@@ -328,182 +348,108 @@ __global__ void __launch_bounds__(32 * TH) conv3x3_mma(const bf16* __restrict__ 
         z1 += bias[co + 1];
       }
       if constexpr (EPI == EPI_F32) {
-        out32[pix * COUT + co] = z0;
-        out32[pix * COUT + co + 1] = z1;
+        *reinterpret_cast<float2*>(out32 + pix * COUT + co) = c2(z0, z1);
       } else {
-        out32[pix * COUT + co] = __bfloat162float(__float2bfloat16(z0));
-        out32[pix * COUT + co + 1] = __bfloat162float(__float2bfloat16(z1));
+        *reinterpret_cast<float2*>(out32 + pix * COUT + co) =
+            c2(__bfloat162float(__float2bfloat16(z0)), __bfloat162float(__float2bfloat16(z1)));
+        *reinterpret_cast<uint32_t*>(out + pix * COUT + co) =
+            relu_mask(pack_bf16(z0, z1), *reinterpret_cast<const uint32_t*>(z + pix * COUT + co));
       }
     }
   }
 }
 
-// Weight gradient dW[tap][co][ci] = sum_p x[p + d(tap)][ci] dy[p][co] for CIN = 32 and COUT = 32 or 8:
-// a persistent grid, each block walking 16 x 8 tiles and warp `tap` accumulating that tap's 32 x 32 (or
-// 8 x 32) block in registers; partial[block] is summed by wgrad_reduce in block order.
-template <int COUT>
-__global__ void __launch_bounds__(32 * NTAP) wgrad_mma(const bf16* __restrict__ x, const bf16* __restrict__ dy, int B,
-                                                       int H, int W, float* __restrict__ partial) {
-  constexpr int CIN = CH;
-  constexpr int XS = TW + 2 + 2;  // smem row stride of the transposed input tile (pixels)
-  constexpr int DS = TW + 8;      // smem row stride of the transposed output-gradient tile
-  __shared__ __align__(16) bf16 s_x[CIN * (TH + 2) * XS];  // [ci][ty][tx]
-  __shared__ __align__(16) bf16 s_dy[COUT * TH * DS];       // [co][ty][tx]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int gid = lane >> 2, tig = lane & 3;
-  const int tap = warp, ky = tap / 3, kx = tap % 3;
-  constexpr int MT = COUT >= 16 ? COUT / 16 : 1;  // M tiles over co (COUT 8: one padded tile)
-  float acc[MT][CIN / 8][4];
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int n = 0; n < CIN / 8; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
-  const int tiles_x = (W + TW - 1) / TW, tiles_y = (H + TH - 1) / TH;
-  const int ntiles = B * tiles_x * tiles_y;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int b = t / (tiles_x * tiles_y), r = t - b * tiles_x * tiles_y;
-    const int y0 = (r / tiles_x) * TH, x0 = (r % tiles_x) * TW;
-    __syncthreads();
-    for (int i = tid; i < (TH + 2) * (TW + 2) * CIN; i += blockDim.x) {
-      const int pix = i / CIN, ci = i - pix * CIN;
-      const int ty = pix / (TW + 2), tx = pix - ty * (TW + 2);
-      const int gy = y0 - 1 + ty, gx = x0 - 1 + tx;
-      bf16 v = __float2bfloat16(0.f);
-      if (gy >= 0 && gy < H && gx >= 0 && gx < W) v = x[(((size_t)b * H + gy) * W + gx) * CIN + ci];
-      s_x[(ci * (TH + 2) + ty) * XS + tx] = v;
-    }
-    for (int i = tid; i < TH * TW * COUT; i += blockDim.x) {
-      const int pix = i / COUT, co = i - pix * COUT;
-      const int ty = pix / TW, tx = pix - ty * TW;
-      const int gy = y0 + ty, gx = x0 + tx;
-      bf16 v = __float2bfloat16(0.f);
-      if (gy < H && gx < W) v = dy[(((size_t)b * H + gy) * W + gx) * COUT + co];
-      s_dy[(co * TH + ty) * DS + tx] = v;
-    }
-    __syncthreads();
-    // K = pixels: one k-step per tile row (16 pixels)
-    for (int ty = 0; ty < TH; ++ty) {
-#pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        uint32_t a[4];
-        const int co0 = m * 16 + gid, co1 = co0 + 8;
-        const bf16* d0 = s_dy + (co0 * TH + ty) * DS + tig * 2;
-        a[0] = *reinterpret_cast<const uint32_t*>(d0);
-        a[2] = *reinterpret_cast<const uint32_t*>(d0 + 8);
-        if (COUT >= 16) {
-          const bf16* d1 = s_dy + (co1 * TH + ty) * DS + tig * 2;
-          a[1] = *reinterpret_cast<const uint32_t*>(d1);
-          a[3] = *reinterpret_cast<const uint32_t*>(d1 + 8);
-        } else {
-          a[1] = a[3] = 0u;  // rows 8..15 of the padded 8-channel tile
-        }
-#pragma unroll
-        for (int n = 0; n < CIN / 8; ++n) {
-          const bf16* xr = s_x + ((n * 8 + gid) * (TH + 2) + ty + ky) * XS + kx + tig * 2;
-          const uint32_t b0 = (uint32_t)__bfloat16_as_ushort(xr[0]) | ((uint32_t)__bfloat16_as_ushort(xr[1]) << 16);
-          const uint32_t b1 = (uint32_t)__bfloat16_as_ushort(xr[8]) | ((uint32_t)__bfloat16_as_ushort(xr[9]) << 16);
-          mma16816(acc[m][n], a, b0, b1);
-        }
-      }
-    }
-  }
-  // partial[block][tap][co][ci]
-  float* pb = partial + ((size_t)blockIdx.x * NTAP + tap) * COUT * CIN;
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int n = 0; n < CIN / 8; ++n)
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int co = m * 16 + gid + 8 * hh;
-        if (co >= COUT) continue;
-        const int ci = n * 8 + tig * 2;
-        pb[co * CIN + ci] = acc[m][n][2 * hh];
-        pb[co * CIN + ci + 1] = acc[m][n][2 * hh + 1];
-      }
-}
-
-// Weight gradient of a 32 -> 32 layer on the tensor cores (tcgen05, kind::f16 BF16, FP32 in TMEM):
-//   dW[ky 3 + kx][co][ci] = sum_p x[p + (ky - 1, kx - 1)][ci] dy[p][co]
-// as D_ky[m = kx 32 + ci][n = co] = sum_k A[m][k] B[n][k] with K = the 16 pixels of one tile row: A is the
-// input tile shifted by kx (rows 96..127 zero), B the output gradient. Per 16 x 8 tile and tile row py,
-// three MMAs (ky = 0, 1, 2: A from halo row py + ky) of M = 128, N = 32, K = 16 into three accumulators
-// (TMEM columns 32 ky). Operands in shared memory in the no-swizzle K-major layout (a core matrix is 8
-// rows x 8 pixels, 16 bytes per row; the tile is staged transposed from the [pixel][channel] activations):
-//   A: [halo row 10][pixel half 2][row group 16][128 B], row group = 4 kx + ci / 8  (LBO 2048, SBO 128)
-//   B: [tile row 8][pixel half 2][channel group 4][128 B]                          (LBO 512, SBO 128)
-// CTAs are persistent over tiles and accumulate in TMEM; each writes partial[block][tap][co][ci], which
-// wgrad_reduce adds in block order.
+// Weight and bias gradient of a layer with 32 input channels on the tensor cores (tcgen05, kind::f16 BF16, FP32 in TMEM):
+//   dW[ky 3 + kx][co][ci] = sum_p x[p + (ky - 1, kx - 1)][ci] dy[p][co],   db[co] = sum_p dy[p][co]
+// as D_ky[m = kx 32 + ci][n = co] = sum_k A[k][m] B[k][n] with K = the 16 pixels of one tile row: A is the input tile
+// shifted by kx, B the output gradient, and row 96 of A is one everywhere, so that row 96 of D is the bias gradient
+// (rows 97 .. 127 are not read). Per 16 x 8 tile and tile row py, three MMAs (ky = 0, 1, 2: A from halo row py + ky) of
+// M = 128, N = NC, K = 16 into three accumulators (TMEM columns NC ky). Both operands are MN-major, as the
+// activations lie in memory: a core matrix is 8 pixels (rows, 16 bytes each) x 8 channels, channel group after
+// channel group kWgGroupA / kWgGroupB apart, pixels 16 bytes apart, so staging is 16-byte copies (the K-major form
+// needed a 2-byte store per value: 57 us a layer at 4 x 320 x 320 against 25; the
+// reduction 11 us against 9). The group strides put the four groups of a
+// pixel in different banks. The next tile is loaded into registers while this tile's MMAs run. CTAs are persistent
+// over tiles and accumulate in TMEM; each writes partial[block][tap][co < COUT][ci] and [co < COUT], which
+// wgrad_sum adds in block order. dy holds NC channels a pixel (COUT of them used).
 constexpr int kWgThreads = 256;
-constexpr uint32_t kWgA = 20 * 2048;  // 40 KB
-constexpr uint32_t kWgB = 16 * 512;   // 8 KB
-constexpr size_t kWgSmem = 1024 + kWgA + kWgB + 64;
+constexpr uint32_t kWgGroupA = 16 * (10 * 16 + 2);  // 2592
+constexpr uint32_t kWgGroupB = 16 * (8 * 16 + 2);   // 2080
+constexpr uint32_t kWgA = 13 * kWgGroupA;           // 12 groups of x, one of ones; groups 13 .. 15 are read past it:
+constexpr uint32_t kWgEnd = 16 * kWgGroupA > kWgA + 4 * kWgGroupB ? 16 * kWgGroupA : kWgA + 4 * kWgGroupB;
+constexpr size_t kWgSmem = 1024 + kWgEnd + 64;
+constexpr int kWgPerSm = 4;  // CTAs per SM: 128 TMEM columns and 43 KB each
 
-__device__ __forceinline__ void st_shared_b16(uint32_t addr, uint16_t v) {
-  asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
-}
-__device__ __forceinline__ uint16_t u4_elem(const uint4& v, int e) {
-  const uint32_t w = e < 2 ? v.x : e < 4 ? v.y : e < 6 ? v.z : v.w;
-  return (uint16_t)((e & 1) ? (w >> 16) : (w & 0xFFFFu));
-}
-
-__global__ void __launch_bounds__(kWgThreads) wgrad_tc(const bf16* __restrict__ x, const bf16* __restrict__ dy, int B,
+template <int NC, int COUT>
+__global__ void __launch_bounds__(kWgThreads, kWgPerSm) wgrad_tc(const bf16* __restrict__ x, const bf16* __restrict__ dy, int B,
                                                        int H, int W, float* __restrict__ partial, int* __restrict__ err) {
+  constexpr uint32_t kCols = NC == 32 ? 128 : 64;
+  constexpr int kX = (TH + 2) * (TW + 2) * 4, kPreX = (kX + kWgThreads - 1) / kWgThreads;
+  constexpr int kD = TH * TW * (NC / 8), kPreD = (kD + kWgThreads - 1) / kWgThreads;
   extern __shared__ unsigned char wg_smem_raw[];
   const uint32_t off = tc::smem_addr(wg_smem_raw);
   unsigned char* sm = wg_smem_raw + ((1024u - (off & 1023u)) & 1023u);
   const uint32_t a_base = tc::smem_addr(sm), b_base = a_base + kWgA;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kWgA + kWgB);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kWgEnd);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ntx = (W + TW - 1) / TW, nty = (H + TH - 1) / TH;
   const int ntiles = ntx * nty * B;
+  auto st16 = [](uint32_t addr, uint4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+  };
   if (tid == 0) {
     tc::mbar_init(bar, 1);
     tc::fence_mbar_init();
   }
-  if (warp == 0) tc::tmem_alloc(tslot, 128);
-  // the zero rows 96..127 of A (row groups 12..15 of every block), written once
-  for (int i = tid; i < 20 * 4 * 8; i += kWgThreads) {
-    const int blk = i >> 5, g = 12 + ((i >> 3) & 3), q = i & 7;
-    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(a_base + (blk * 16 + g) * 128 + q * 16), "r"(0u)
-                 : "memory");
-  }
+  if (warp == 0) tc::tmem_alloc(tslot, kCols);
+  for (int i = tid; i < (TH + 2) * TW; i += kWgThreads)  // the ones: BF16 1 in the group's first channel
+    st16(a_base + 12 * kWgGroupA + 16 * i, make_uint4(0x3F80u, 0u, 0u, 0u));
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
   const bool drop = tc::g_drop_arrival != 0;
-  bool ok = true;
-  int it = 0;
-  for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++it) {
+  uint4 px[kPreX], pd[kPreD];
+  auto fetch = [&](int t) {
     const int bx = t % ntx, by = (t / ntx) % nty, b = t / (ntx * nty);
     const int x0 = bx * TW, y0 = by * TH;
-    // x halo tile -> A, transposed and shifted: item (halo row, halo column, channel group of 8)
-    for (int i = tid; i < (TH + 2) * (TW + 2) * 4; i += kWgThreads) {
-      const int cg = i & 3, col = (i >> 2) % (TW + 2), hy = (i >> 2) / (TW + 2);
+#pragma unroll
+    for (int j = 0; j < kPreX; ++j) {  // item (halo row, halo column, channel group)
+      const int i = tid + j * kWgThreads, cg = i & 3, col = (i >> 2) % (TW + 2), hy = (i >> 2) / (TW + 2);
       const int gy = y0 + hy - 1, gx = x0 + col - 1;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gy >= 0 && gy < H && gx >= 0 && gx < W)
-        v = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)b * H + gy) * W + gx) * CH) + cg);
-#pragma unroll
-      for (int kx = 0; kx < 3; ++kx) {
-        const int px = col - kx;
-        if (px < 0 || px >= TW) continue;
-        const uint32_t base = a_base + ((hy * 2 + (px >> 3)) * 16 + kx * 4 + cg) * 128 + (px & 7) * 2;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) st_shared_b16(base + e * 16, u4_elem(v, e));
-      }
+      px[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < kX && gy >= 0 && gy < H && gx >= 0 && gx < W)
+        px[j] = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)b * H + gy) * W + gx) * CH) + cg);
     }
-    // dy tile -> B, transposed: item (tile row, pixel, channel group)
-    for (int i = tid; i < TH * TW * 4; i += kWgThreads) {
-      const int cg = i & 3, px = (i >> 2) % TW, py = (i >> 2) / TW;
-      const int gy = y0 + py, gx = x0 + px;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gy < H && gx < W) v = __ldg(reinterpret_cast<const uint4*>(dy + (((size_t)b * H + gy) * W + gx) * CH) + cg);
-      const uint32_t base = b_base + ((py * 2 + (px >> 3)) * 4 + cg) * 128 + (px & 7) * 2;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) st_shared_b16(base + e * 16, u4_elem(v, e));
+    for (int j = 0; j < kPreD; ++j) {  // item (tile row, pixel, channel group)
+      const int i = tid + j * kWgThreads, cg = i % (NC / 8), p = i / (NC / 8);
+      const int gy = y0 + p / TW, gx = x0 + p % TW;
+      pd[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < kD && gy < H && gx < W)
+        pd[j] = __ldg(reinterpret_cast<const uint4*>(dy + (((size_t)b * H + gy) * W + gx) * NC) + cg);
+    }
+  };
+  bool ok = true;
+  int it = 0;
+  if ((int)blockIdx.x < ntiles) fetch(blockIdx.x);
+  for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++it) {
+    // the operand buffers are free (the previous tile's MMAs are done)
+#pragma unroll
+    for (int j = 0; j < kPreX; ++j) {
+      const int i = tid + j * kWgThreads, cg = i & 3, col = (i >> 2) % (TW + 2), hy = (i >> 2) / (TW + 2);
+      if (i < kX)
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx) {
+          const int p = col - kx;
+          if (p >= 0 && p < TW) st16(a_base + (kx * 4 + cg) * kWgGroupA + 16 * (hy * TW + p), px[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kPreD; ++j) {
+      const int i = tid + j * kWgThreads, cg = i % (NC / 8), p = i / (NC / 8);
+      if (i < kD) st16(b_base + cg * kWgGroupB + 16 * p, pd[j]);
     }
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -511,33 +457,36 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc(const bf16* __restrict__ 
     tc::fence_after_sync();
     // (the test hook withholds block 0's first tile: no MMAs and no commit, so the wait below runs out)
     if (tid == 0 && !(it == 0 && blockIdx.x == 0 && drop)) {
-      const uint32_t idesc = tc::idesc_bf16(128, CH);
+      const uint32_t idesc = tc::idesc_bf16(128, NC) | (1u << 15) | (1u << 16);  // both operands MN-major
       for (int py = 0; py < TH; ++py)
         for (int ky = 0; ky < 3; ++ky)
-          tc::mma_bf16(tmem + 32 * ky, tc::desc_interleave(a_base + (py + ky) * 2 * 2048, 2048, 128),
-                       tc::desc_interleave(b_base + py * 2 * 512, 512, 128), idesc, (it > 0 || py > 0) ? 1u : 0u);
+          tc::mma_bf16(tmem + NC * ky, tc::desc_interleave(a_base + (py + ky) * (16 * TW), 128, kWgGroupA),
+                       tc::desc_interleave(b_base + py * (16 * TW), 128, kWgGroupB), idesc, (it > 0 || py > 0) ? 1u : 0u);
       tc::mma_commit(bar);
     }
+    if (t + (int)gridDim.x < ntiles) fetch(t + gridDim.x);
     ok = tc::mbar_wait(bar, it & 1);
     if (!ok) tc::mbar_wait(bar, it & 1);  // wait (bounded) for MMAs still in flight before the tiles are reused
     tc::fence_after_sync();
     ok = __syncthreads_and(ok);
   }
-  // epilogue: TMEM lane m = kx 32 + ci (warps 0..3 own lanes 32 w .. 32 w + 31), column 32 ky + co
+  // epilogue: TMEM lane m (warps 0..3 own lanes 32 w .. 32 w + 31), column NC ky + co
   if (ok && warp < 4) {
     const int m = 32 * warp + lane;
     const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16);
-    float* pb = partial + (size_t)blockIdx.x * NTAP * CH * CH;
+    float* pb = partial + (size_t)blockIdx.x * (NTAP * COUT * CH + COUT);
 #pragma unroll
     for (int ky = 0; ky < 3; ++ky) {
       float v[16];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        tc::tmem_ld16(taddr + 32 * ky + 16 * h, v);
-        if (m < 96) {
-          const int kx = m >> 5, ci = m & 31, tap = ky * 3 + kx;
+      for (int h = 0; h < NC / 16; ++h) {
+        tc::tmem_ld16(taddr + NC * ky + 16 * h, v);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) pb[((size_t)tap * CH + 16 * h + j) * CH + ci] = v[j];
+        for (int j = 0; j < 16; ++j) {
+          const int co = 16 * h + j;
+          if (co >= COUT) continue;
+          if (m < 96) pb[((size_t)(ky * 3 + (m >> 5)) * COUT + co) * CH + (m & 31)] = v[j];
+          if (m == 96 && ky == 0) pb[NTAP * COUT * CH + co] = v[j];
         }
       }
     }
@@ -547,59 +496,28 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc(const bf16* __restrict__ 
   __syncthreads();
   if (warp == 0) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem, 128);
+    tc::tmem_dealloc(tmem, kCols);
   }
 }
 
-// Two-level fixed-order sum of partial[b][i] over the blocks b: stage 1 adds block range s (blockIdx.y) into
-// tmp[s][i], stage 2 (wgrad_reduce with nblocks = the range count) adds the ranges in order.
-constexpr int kWgRanges = 16;
-__global__ void wgrad_reduce_ranges(const float* __restrict__ partial, int nblocks, int n, float* __restrict__ tmp) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
-  if (i >= n) return;
-  const int b0 = (int)((long long)r * nblocks / gridDim.y), b1 = (int)((long long)(r + 1) * nblocks / gridDim.y);
+// grad[i] = sum over the blocks b of partial[b][i], in a fixed order: a block takes 32 outputs, each of its 16 warps
+// a range of b in order, and the warps' sums are added in order.
+constexpr int kWgSumWarps = 16;
+__global__ void __launch_bounds__(32 * kWgSumWarps) wgrad_sum(const float* __restrict__ partial, int nblocks, int n,
+                                                              float* __restrict__ grad) {
+  __shared__ float sh[kWgSumWarps][32];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  const int b0 = r * nblocks / kWgSumWarps, b1 = (r + 1) * nblocks / kWgSumWarps;
   float s = 0.f;
-  for (int b = b0; b < b1; ++b) s += partial[(size_t)b * n + i];
-  tmp[(size_t)r * n + i] = s;
-}
-
-// grad[i] = sum_b partial[b][i] (block order)
-__global__ void wgrad_reduce(const float* __restrict__ partial, int nblocks, int n, float* __restrict__ grad) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * n + i];
-    grad[i] = s;
+  if (i < n) {
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b) s += partial[(size_t)b * n + i];
   }
-}
-
-// Per-channel sums of dy [npix][C] (the bias gradient), stage 1: block b sums the pixels of its contiguous
-// chunk -- C / 2 threads per pixel, two channels each, so that a warp reads consecutive bytes -- and writes
-// partial[b][C]; sum_partials adds the blocks' partials in block order (deterministic).
-template <int C>
-__global__ void __launch_bounds__(256) bias_grad_partial(const bf16* __restrict__ dy, size_t npix,
-                                                         float* __restrict__ partial) {
-  constexpr int TPP = C / 2, PPB = 256 / TPP;  // threads per pixel, pixels per pass
-  __shared__ float2 sh[256];
-  const int t = threadIdx.x, cp = t % TPP, pr = t / TPP;
-  const size_t chunk = (npix + gridDim.x - 1) / gridDim.x;
-  const size_t p0 = (size_t)blockIdx.x * chunk, p1 = min(npix, p0 + chunk);
-  float2 acc = c2(0.f, 0.f);
-  for (size_t p = p0 + pr; p < p1; p += PPB) {
-    const __nv_bfloat162 v = reinterpret_cast<const __nv_bfloat162*>(dy + p * C)[cp];
-    acc.x += __low2float(v);
-    acc.y += __high2float(v);
-  }
-  sh[t] = acc;
+  sh[r][lane] = s;
   __syncthreads();
-  if (t < TPP) {
-    float2 a = c2(0.f, 0.f);
-    for (int r = 0; r < PPB; ++r) {
-      a.x += sh[r * TPP + t].x;
-      a.y += sh[r * TPP + t].y;
-    }
-    partial[(size_t)blockIdx.x * C + 2 * t] = a.x;
-    partial[(size_t)blockIdx.x * C + 2 * t + 1] = a.y;
-  }
+  if (r || i >= n) return;
+  for (int q = 1; q < kWgSumWarps; ++q) s += sh[q][lane];
+  grad[i] = s;
 }
 
 // out[i] = sum over blocks b of partial[b * stride + i], i < n: one CUDA block per output, its 128 threads
@@ -620,15 +538,21 @@ __global__ void __launch_bounds__(128) sum_partials(const float* __restrict__ pa
   if (threadIdx.x == 0) out[i] = sh[0];
 }
 
-// w'[tap'][ci][co] = w[8 - tap'][co][ci] (padded to COP output / CIP input channels) for the data gradient.
-__global__ void flip_transpose(const bf16* __restrict__ w, int cout, int cin, int cop, int cip, bf16* __restrict__ wt) {
-  const int n = NTAP * cip * cop;
+// The data gradients' weights of layers 1 .. 7 (blockIdx.y = layer - 1): w'[tap'][ci][co] = w[8 - tap'][co][ci], the
+// output layer's 8 output channels padded to 16. w: the flat BF16 parameters, layer l's weights at at[l - 1].
+struct LayerOffsets {
+  int at[7];
+};
+__global__ void flip_transpose(const bf16* __restrict__ w, LayerOffsets o, bf16* __restrict__ wt) {
+  const int l = blockIdx.y, cout = l == 6 ? 8 : CH, cop = l == 6 ? 16 : CH, n = NTAP * CH * cop;
+  const bf16* wl = w + o.at[l];
+  bf16* out = wt + (size_t)l * NTAP * CH * CH;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int tap = i / (cip * cop), r = i - tap * cip * cop;
+    const int tap = i / (CH * cop), r = i - tap * CH * cop;
     const int ci = r / cop, co = r - ci * cop;  // wt[tap][ci (as out)][co (as in)]
     bf16 v = __float2bfloat16(0.f);
-    if (ci < cin && co < cout) v = w[((size_t)(8 - tap) * cout + co) * cin + ci];
-    wt[i] = v;
+    if (co < cout) v = wl[((size_t)(8 - tap) * cout + co) * CH + ci];
+    out[i] = v;
   }
 }
 
@@ -753,77 +677,38 @@ __global__ void __launch_bounds__(32 * kConvInWarps) conv_in_wgrad_partial(const
   }
 }
 
-// g = bf16(acc) * relu'(z): the residual stream's FP32 gradient rounded to BF16 (the same rounding as a
-// separate conversion) and masked by the ReLU's derivative, four channels per thread, and with `partial` the
-// per-channel sums of g over the block's contiguous pixels (the bias gradient, which otherwise reads g again:
-// 10 us a layer at 4 x 320 x 320): partial[block][CH], added in block order by sum_partials.
-__global__ void __launch_bounds__(256) relu_bwd_acc(const float* __restrict__ acc, const bf16* __restrict__ z, size_t npix,
-                                                    bf16* __restrict__ g, float* __restrict__ partial) {
-  __shared__ float4 sh[256];
-  const int t = threadIdx.x;
-  const size_t chunk = (npix + gridDim.x - 1) / gridDim.x;
-  const size_t i1 = min(npix, (blockIdx.x + 1) * chunk) * (CH / 4);
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-  for (size_t i = (size_t)blockIdx.x * chunk * (CH / 4) + t; i < i1; i += 256) {
-    const float4 a = reinterpret_cast<const float4*>(acc)[i];
-    const uint2 zz = reinterpret_cast<const uint2*>(z)[i];
-    const __nv_bfloat162 z01 = *reinterpret_cast<const __nv_bfloat162*>(&zz.x);
-    const __nv_bfloat162 z23 = *reinterpret_cast<const __nv_bfloat162*>(&zz.y);
-    const bf16 zero = __float2bfloat16(0.f);
-    const bf16 g0 = __bfloat162float(z01.x) > 0.f ? __float2bfloat16(a.x) : zero;
-    const bf16 g1 = __bfloat162float(z01.y) > 0.f ? __float2bfloat16(a.y) : zero;
-    const bf16 g2 = __bfloat162float(z23.x) > 0.f ? __float2bfloat16(a.z) : zero;
-    const bf16 g3 = __bfloat162float(z23.y) > 0.f ? __float2bfloat16(a.w) : zero;
-    uint2 o;
-    __nv_bfloat162 o01, o23;
-    o01.x = g0;
-    o01.y = g1;
-    o23.x = g2;
-    o23.y = g3;
-    o.x = *reinterpret_cast<const uint32_t*>(&o01);
-    o.y = *reinterpret_cast<const uint32_t*>(&o23);
-    reinterpret_cast<uint2*>(g)[i] = o;
-    s.x += __bfloat162float(g0);
-    s.y += __bfloat162float(g1);
-    s.z += __bfloat162float(g2);
-    s.w += __bfloat162float(g3);
-  }
-  if (!partial) return;
-  sh[t] = s;  // channels 4 (t % 8) ..
-  __syncthreads();
-  if (t < CH / 4) {
-    float4 a = sh[t];
-    for (int r = 1; r < 256 / (CH / 4); ++r) {
-      const float4 b = sh[r * (CH / 4) + t];
-      a.x += b.x;
-      a.y += b.y;
-      a.z += b.z;
-      a.w += b.w;
-    }
-    reinterpret_cast<float4*>(partial + (size_t)blockIdx.x * CH)[t] = a;
-  }
-}
-
 __global__ void to_bf16(const float* __restrict__ a, size_t n, bf16* __restrict__ out) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = __float2bfloat16(a[i]);
 }
 
-// Mean squared error over the 6 used output channels and its gradient (padded to 8 channels, BF16).
+// Mean squared error over the 6 used output channels and its gradient (BF16, padded to the 16 channels the
+// tensor-core kernels take).
 __global__ void mse_loss(const float* __restrict__ y, const float* __restrict__ t, size_t npix, float scale,
                          bf16* __restrict__ g, double* __restrict__ partial) {
   __shared__ double sh[256];
   double s = 0;
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x) {
-    for (int c = 0; c < 8; ++c) {
-      float d = 0.f;
-      if (c < 6) {
-        d = y[p * 8 + c] - t[p * 6 + c];
-        s += (double)d * d;
-      }
-      g[p * 8 + c] = __float2bfloat16(2.f * d * scale);
-    }
+    float d[8];
+    const float4 ya = reinterpret_cast<const float4*>(y)[2 * p], yb = reinterpret_cast<const float4*>(y)[2 * p + 1];
+    const float2* tp = reinterpret_cast<const float2*>(t) + 3 * p;
+    const float2 t0 = tp[0], t1 = tp[1], t2 = tp[2];
+    d[0] = ya.x - t0.x;
+    d[1] = ya.y - t0.y;
+    d[2] = ya.z - t1.x;
+    d[3] = ya.w - t1.y;
+    d[4] = yb.x - t2.x;
+    d[5] = yb.y - t2.y;
+    d[6] = d[7] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) s += (double)d[c] * d[c];
+    uint4 o;
+    o.x = pack_bf16(2.f * d[0] * scale, 2.f * d[1] * scale);
+    o.y = pack_bf16(2.f * d[2] * scale, 2.f * d[3] * scale);
+    o.z = pack_bf16(2.f * d[4] * scale, 2.f * d[5] * scale);
+    o.w = 0u;
+    reinterpret_cast<uint4*>(g)[2 * p] = o;
+    reinterpret_cast<uint4*>(g)[2 * p + 1] = make_uint4(0u, 0u, 0u, 0u);
   }
   sh[threadIdx.x] = s;
   __syncthreads();
@@ -981,7 +866,10 @@ class WarmStartCnn {
       // all of the unified L1 / shared storage as shared memory, so that several CTAs fit on an SM
       PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     }
-    PDT_CUDA_CHECK(cudaFuncSetAttribute(wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
+    for (auto fn : {wgrad_tc<32, 32>, wgrad_tc<16, 8>}) {
+      PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
+      PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    }
     err_.ensure(sizeof(int));
     PDT_CUDA_CHECK(cudaMemset(err_.p, 0, sizeof(int)));
     int dev = 0;
@@ -1046,7 +934,8 @@ class WarmStartCnn {
       PDT_LAUNCH_CHECK();
       count_launch();
     }
-    conv3x3_mma<CH, 8, EPI_F32><<<grid, 32 * TH, 0, st>>>(h_[6].as<bf16>(), W_[7].wb, B_[7].w, H, W, o_.as<float>());
+    conv3x3_mma<CH, 8, EPI_F32><<<grid, 32 * TH, 0, st>>>(h_[6].as<bf16>(), W_[7].wb, B_[7].w, H, W, o_.as<float>(),
+                                                          nullptr, nullptr);
     PDT_LAUNCH_CHECK();
     count_launch();
   }
@@ -1058,49 +947,42 @@ class WarmStartCnn {
     const int lb = grid_for(npix);
     part_.ensure(sizeof(double) * lb);
     mse_loss<<<lb, 256, 0, st>>>(o_.as<float>(), target, npix, scale, go_.as<bf16>(), part_.as<double>());
+    LayerOffsets at;
+    for (int l = 1; l <= 7; ++l) at.at[l - 1] = (int)(W_[l].wb - pb_.as<bf16>());
+    flip_transpose<<<dim3(36, 7), 256, 0, st>>>(pb_.as<bf16>(), at, wt_.as<bf16>());
+    auto wt = [&](int l) { return wt_.as<bf16>() + (size_t)(l - 1) * NTAP * CH * CH; };
     PDT_LAUNCH_CHECK();
-    count_launch();
     const dim3 grid((W + TW - 1) / TW, (H + TH - 1) / TH, B);
     const int tgrid = conv_tc_grid(B, H, W);
-    // conv_out: dW, db, and dh6 = conv(go, W7') (8 -> 32 channels, padded to 16 input channels)
+    // conv_out: dW, db, and dh6 = conv(go, W7') (8 -> 32 channels, padded to 16 input channels), with which the
+    // residual stream's FP32 gradient starts as G = dh6 (the BF16 rounding of the convolution's output)
     wgrad(8, h_[6].as<bf16>(), go_.as<bf16>(), B, H, W, W_[7].g, st);
-    bias_gradient(go_.as<bf16>(), npix, B_[7].g, st);
-    // go is [npix][8]; the data-gradient kernel needs 16 input channels: pad into go16_
-    pad8to16(go_.as<bf16>(), npix, st);
-    flip_transpose<<<64, 256, 0, st>>>(W_[7].wb, 8, CH, 16, CH, wt_.as<bf16>());
+    bf16* gz = gz_[0].as<bf16>();  // dz = G * relu'(z_l) of the layer at hand; the next layer's goes to the other buffer
+    bf16* gn = gz_[1].as<bf16>();
+    conv3x3_mma<16, CH, EPI_F32_BF16><<<grid, 32 * TH, 0, st>>>(go_.as<bf16>(), wt(7), nullptr, H, W, gacc_.as<float>(),
+                                                                z_[6].as<bf16>(), gz);
     PDT_LAUNCH_CHECK();
-    // the residual stream's FP32 gradient starts as G = dh6 (the BF16 rounding of the convolution's output)
-    conv3x3_mma<16, CH, EPI_F32_BF16><<<grid, 32 * TH, 0, st>>>(go16_.as<bf16>(), wt_.as<bf16>(), nullptr, H, W,
-                                                                gacc_.as<float>());
-    PDT_LAUNCH_CHECK();
-    count_launch(3);  // mse_loss, flip_transpose, conv3x3_mma (the bias gradient counts its own)
+    count_launch(3);  // mse_loss, flip_transpose, conv3x3_mma
     for (int l = 6; l >= 1; --l) {
-      // h_l = h_{l-1} + relu(z_l), z_l = conv_l(h_{l-1}):  dz = G * relu'(z_l); dh_{l-1} = G + conv_l^T(dz)
-      const int nb = kPartialBlocksPerSm * sms_;
-      bpart_.ensure(sizeof(float) * (size_t)nb * kConvInPartial);
-      relu_bwd_acc<<<nb, 256, 0, st>>>(gacc_.as<float>(), z_[l].as<bf16>(), npix, gz_.as<bf16>(), bpart_.as<float>());
-      sum_partials<<<CH, 128, 0, st>>>(bpart_.as<float>(), nb, CH, CH, B_[l].g);
+      // h_l = h_{l-1} + relu(z_l), z_l = conv_l(h_{l-1}):  dh_{l-1} = G + conv_l^T(dz), added into the FP32 residual
+      // gradient in the convolution's epilogue, which also masks it for the layer below
+      wgrad(CH, h_[l - 1].as<bf16>(), gz, B, H, W, W_[l].g, st);
+      conv3x3_tc<EPI_ACC><<<tgrid, kConvTcThreads, kConvTcSmem, st>>>(gz, wt(l), nullptr, B, H, W, gn, z_[l - 1].as<bf16>(),
+                                                                    err_.as<int>(), gacc_.as<float>());
       PDT_LAUNCH_CHECK();
-      wgrad(CH, h_[l - 1].as<bf16>(), gz_.as<bf16>(), B, H, W, W_[l].g, st);
-      flip_transpose<<<64, 256, 0, st>>>(W_[l].wb, CH, CH, CH, CH, wt_.as<bf16>());
-      // dh_{l-1} += conv_l^T(dz), added into the FP32 residual gradient in the convolution's epilogue
-      conv3x3_tc<EPI_ACC><<<tgrid, kConvTcThreads, kConvTcSmem, st>>>(gz_.as<bf16>(), wt_.as<bf16>(), nullptr, B, H, W,
-                                                                    nullptr, nullptr, err_.as<int>(), gacc_.as<float>());
-      PDT_LAUNCH_CHECK();
-      count_launch(4);  // relu_bwd_acc, sum_partials, flip_transpose, conv3x3_tc
+      count_launch();
+      std::swap(gz, gn);
     }
-    // conv_in: h1 = relu(z_0): dz0 = G * relu'(z0)
+    // conv_in: h1 = relu(z_0)
     {
       const int nb = kPartialBlocksPerSm * sms_;
-      relu_bwd_acc<<<nb, 256, 0, st>>>(gacc_.as<float>(), z_[0].as<bf16>(), npix, gz_.as<bf16>(), nullptr);
       bpart_.ensure(sizeof(float) * (size_t)nb * kConvInPartial);
-      conv_in_wgrad_partial<<<nb, 32 * kConvInWarps, 0, st>>>(x_.as<float>(), gz_.as<bf16>(), B, H, W,
-                                                              bpart_.as<float>());
+      conv_in_wgrad_partial<<<nb, 32 * kConvInWarps, 0, st>>>(x_.as<float>(), gz, B, H, W, bpart_.as<float>());
       // the weights and, right behind them as in the flat gradient, the biases
       sum_partials<<<kConvInPartial, 128, 0, st>>>(bpart_.as<float>(), nb, kConvInPartial, kConvInPartial, W_[0].g);
       PDT_LAUNCH_CHECK();
     }
-    count_launch(3);  // relu_bwd_acc, conv_in_wgrad_partial, sum_partials
+    count_launch(2);  // conv_in_wgrad_partial, sum_partials
     std::vector<double> h(lb);
     PDT_CUDA_CHECK(cudaMemcpyAsync(h.data(), part_.p, sizeof(double) * lb, cudaMemcpyDeviceToHost, st));
     PDT_CUDA_CHECK(cudaStreamSynchronize(st));
@@ -1179,56 +1061,35 @@ class WarmStartCnn {
       z_[l].ensure(npix * CH * sizeof(bf16));
     }
     o_.ensure(npix * 8 * sizeof(float));
-    go_.ensure(npix * 8 * sizeof(bf16));
-    go16_.ensure(npix * 16 * sizeof(bf16));
-    gz_.ensure(npix * CH * sizeof(bf16));
+    go_.ensure(npix * 16 * sizeof(bf16));
+    for (auto& g : gz_) g.ensure(npix * CH * sizeof(bf16));
     gacc_.ensure(npix * CH * sizeof(float));
-    wt_.ensure(NTAP * CH * CH * sizeof(bf16));
+    wt_.ensure((size_t)7 * NTAP * CH * CH * sizeof(bf16));
     B_n_ = B;
     H_n_ = H;
     W_n_ = W;
   }
-  void pad8to16(const bf16* g8, size_t npix, cudaStream_t st) {
-    PDT_CUDA_CHECK(cudaMemsetAsync(go16_.p, 0, npix * 16 * sizeof(bf16), st));
-    PDT_CUDA_CHECK(cudaMemcpy2DAsync(go16_.p, 16 * sizeof(bf16), g8, 8 * sizeof(bf16), 8 * sizeof(bf16), npix,
-                                     cudaMemcpyDeviceToDevice, st));
-  }
+  // The weight gradient and, behind it in the flat array, the bias gradient of a layer.
   void wgrad(int cout, const bf16* x, const bf16* dy, int B, int H, int W, float* grad, cudaStream_t st) {
-    int sms = 0, dev = 0;
-    PDT_CUDA_CHECK(cudaGetDevice(&dev));
-    PDT_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int tiles = B * ((W + TW - 1) / TW) * ((H + TH - 1) / TH);
-    // the tensor-core kernel: three persistent CTAs per SM (128 TMEM columns, 50 KB shared memory each)
-    const int nb = std::max(1, std::min(sms * (cout == CH ? 3 : 2), tiles));
-    const int n = NTAP * cout * CH;
-    wpart_.ensure((size_t)std::max(1, std::min(sms * 3, tiles)) * NTAP * CH * CH * sizeof(float));
+    const int nb = std::max(1, std::min(sms_ * kWgPerSm, tiles));
+    const int n = NTAP * cout * CH + cout;
+    wpart_.ensure((size_t)nb * (NTAP * CH * CH + CH) * sizeof(float));
     if (cout == CH)
-      wgrad_tc<<<nb, kWgThreads, kWgSmem, st>>>(x, dy, B, H, W, wpart_.as<float>(), err_.as<int>());
+      wgrad_tc<32, 32><<<nb, kWgThreads, kWgSmem, st>>>(x, dy, B, H, W, wpart_.as<float>(), err_.as<int>());
     else
-      wgrad_mma<8><<<nb, 32 * NTAP, 0, st>>>(x, dy, B, H, W, wpart_.as<float>());
+      wgrad_tc<16, 8><<<nb, kWgThreads, kWgSmem, st>>>(x, dy, B, H, W, wpart_.as<float>(), err_.as<int>());
     PDT_LAUNCH_CHECK();
-    wtmp_.ensure(sizeof(float) * (size_t)kWgRanges * NTAP * CH * CH);
-    wgrad_reduce_ranges<<<dim3((n + 255) / 256, kWgRanges), 256, 0, st>>>(wpart_.as<float>(), nb, n, wtmp_.as<float>());
-    wgrad_reduce<<<grid_for(n), 256, 0, st>>>(wtmp_.as<float>(), kWgRanges, n, grad);
+    wgrad_sum<<<(n + 31) / 32, 32 * kWgSumWarps, 0, st>>>(wpart_.as<float>(), nb, n, grad);
     PDT_LAUNCH_CHECK();
-    count_launch(3);
+    count_launch(2);
   }
 
   CnnParam W_[kLayers], B_[kLayers];
   size_t total_ = 0;
   DevBuf pw_, pg_, pm_, pv_, pb_;  // flat FP32 master weights, gradients, Adam moments; BF16 copy
-  DevBuf x_, h_[7], z_[7], o_, go_, go16_, gz_, gacc_, wt_, wpart_, part_, t_, sc_, err_, bpart_, wtmp_;
+  DevBuf x_, h_[7], z_[7], o_, go_, gz_[2], gacc_, wt_, wpart_, part_, t_, sc_, err_, bpart_;
 
-  // Bias gradient db[c] = sum over pixels of dy[p][c] of the 8-channel output layer: chunked partial sums, then
-  // the partials in block order.
-  void bias_gradient(const bf16* dy, size_t npix, float* db, cudaStream_t st) {
-    const int nb = 2 * sms_;
-    bpart_.ensure(sizeof(float) * (size_t)kPartialBlocksPerSm * sms_ * kConvInPartial);
-    bias_grad_partial<8><<<nb, 256, 0, st>>>(dy, npix, bpart_.as<float>());
-    sum_partials<<<8, 128, 0, st>>>(bpart_.as<float>(), nb, 8, 8, db);
-    PDT_LAUNCH_CHECK();
-    count_launch(2);
-  }
   int sms_ = 1;
   int conv_tc_per_sm_ = 8;  // resident conv3x3_tc CTAs per SM (each holds 32 TMEM columns: 8 x 32 <= 512)
   int B_n_ = 0, H_n_ = 0, W_n_ = 0;
