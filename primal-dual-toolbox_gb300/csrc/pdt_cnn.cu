@@ -30,21 +30,13 @@ namespace {
 typedef __nv_bfloat16 bf16;
 
 constexpr int CH = 32;    // hidden channels
-constexpr int TW = 16;    // pixel tile width (one mma M tile)
-constexpr int TH = 8;     // pixel tile height (one row per warp)
+constexpr int TW = 16;    // the weight gradients' pixel tile: K = TW pixels an MMA
+constexpr int TH = 8;
 constexpr int NTAP = 9;
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
-}
-
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // The pair of BF16 values g where the pair z is positive, else zero.
@@ -61,148 +53,187 @@ enum Epi {
   EPI_F32_BF16 = 5   // out32 = bf16(z), stored as FP32 (starts a residual stream's gradient), and out likewise
 };
 
-// 32 -> 32 channel 3 x 3 convolution on the fifth-generation tensor cores (tcgen05 kind::f16, BF16
-// operands, FP32 accumulator in tensor memory), as an implicit GEMM without an im2col copy. One CTA computes
-// a tile of 8 x 16 pixels (x, y) = the 128 rows of one MMA tile, rows ordered y-major. The input tile with
-// its one-pixel zero halo (10 x 18 pixels) sits in shared memory in the no-swizzle K-major layout: channel
-// group g (8 channels, 16 bytes) of pixel p at byte g 2912 + 16 p, so eight consecutive pixels form a core
-// matrix (the group stride, two pixels more than the 180 of a group, puts the four groups of a pixel in
-// four different bank quarters, so the halo's 16-byte stores do not conflict); the 8-pixel groups of the M tile are one halo row (160 bytes) apart, and tap (ky, kx) is the
-// same layout started 16 (10 ky + kx) bytes in. The weights sit the same way ([tap][g][co] x 16 bytes).
-// K = (tap, channel) = 288 in 18 MMAs of K = 16 (two channel groups), N = 32 output channels. One thread
-// issues the MMAs and commits them to an mbarrier; the epilogue reads pixel rows from tensor memory
-// (warps q and q + 4 share lane quarter q, 16 output channels each).
+// 3 x 3 convolution of CIN = 32 or 16 to COUT = 32 or 8 channels on the fifth-generation tensor cores (tcgen05
+// kind::f16, BF16 operands, FP32 accumulator in tensor memory), as an implicit GEMM without an im2col copy: the
+// hidden layers, their data gradients, the output layer (its 8 channels padded to N = 16) and the output layer's data
+// gradient (16 padded input channels). One CTA computes a tile of 8 x 16 pixels (x, y) = the 128 rows of one MMA tile,
+// rows ordered y-major. The input tile with its one-pixel zero halo (10 x 18 pixels) sits in shared memory in the
+// no-swizzle K-major layout: channel group g (8 channels, 16 bytes) of pixel p at byte g kGroup + 16 p, so eight
+// consecutive pixels form a core matrix (four groups are two pixels further apart, which puts the groups of a pixel in
+// different bank quarters, so the halo's 16-byte stores do not conflict); the 8-pixel groups of the M tile are one
+// halo row (160 bytes) apart, and tap (ky, kx) is the same layout started 16 (10 ky + kx) bytes in. The weights sit
+// the same way ([tap][g][co] x 16 bytes). K = (tap, channel) in MMAs of K = 16 (two channel groups). One thread issues
+// the MMAs and commits them to an mbarrier; the epilogue reads pixel rows from tensor memory (warps q and q + 4 share
+// lane quarter q, and half the output channels each).
 constexpr int kConvTcThreads = 256;
 constexpr int kConvTcTW = 8, kConvTcTH = 16;                      // tile: 8 pixels wide, 16 rows
 constexpr int kConvTcHaloPix = (kConvTcTW + 2) * (kConvTcTH + 2);  // 180
-constexpr uint32_t kConvTcGroup = 16 * (kConvTcHaloPix + 2);       // 2912: one channel group of the tile
-constexpr uint32_t kConvTcIn = 4 * kConvTcGroup;                   // 11,648 bytes
-constexpr uint32_t kConvTcW = NTAP * 4 * 32 * 16;                   // 18,432 bytes
-// The farthest operand byte an MMA reads: A at tap (2, 2), channel groups 2, 3: 16 (2 10 + 2) + 2 2912 +
-// 2912 (second K core matrix) + 15 160 (last 8-pixel group) + 128 = 11,616 <= kConvTcIn; B at tap 8, groups
-// 2, 3: (8 4 + 2) 512 + 512 + 3 128 + 128 = 18,432 = kConvTcW. The mbarrier, the tensor-memory slot and
-// the 32 biases (FP32) follow the weights.
-constexpr size_t kConvTcSmem = 1024 + kConvTcIn + kConvTcW + 16 + 128;
-constexpr int kConvTcItems = kConvTcHaloPix * 4;                                 // 720 16-byte items per tile
-constexpr int kConvTcPre = (kConvTcItems + kConvTcThreads - 1) / kConvTcThreads;  // 3 per thread
+constexpr int kConvTcBufs = 3;
+
+template <int CIN, int COUT>
+struct ConvTc {
+  static constexpr int kGroups = CIN / 8, kN = COUT < 16 ? 16 : COUT;
+  static constexpr uint32_t kGroup = 16 * (kConvTcHaloPix + (kGroups == 4 ? 2 : 0));  // one channel group of the tile
+  static constexpr uint32_t kIn = kGroups * kGroup, kW = NTAP * kGroups * kN * 16;
+  // The farthest operand byte an MMA reads: A at tap (2, 2), the last two channel groups: 16 (2 10 + 2) +
+  // (kGroups - 1) kGroup + 15 160 (last 8-pixel group) + 128 = (kGroups - 1) kGroup + 2880 <= kIn; B at tap 8, the last
+  // two groups: the end of its kN rows, kW. Two mbarriers, the tensor-memory slot and the kN biases (FP32) follow.
+  static constexpr size_t kSmem = 1024 + kConvTcBufs * kIn + kW + 32 + 4 * kN;
+  static constexpr int kItems = kConvTcHaloPix * kGroups;                             // 16-byte items per tile
+  static constexpr int kPre = (kItems + kConvTcThreads - 1) / kConvTcThreads;  // per thread
+  static constexpr uint32_t kCols = 2 * kN < 32 ? 32 : 2 * kN;                         // two accumulators
+};
 
 __device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&v)[4]) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
 }
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 
 // Persistent: a CTA loads the weights once and walks tiles t = blockIdx.x, + gridDim.x, ... of the
-// (x tiles) x (y tiles) x B grid; the completion barrier's phase alternates per tile. The next tile's halo
-// is loaded into registers right after this tile's MMAs are issued, so its global-load latency overlaps
-// the MMAs and the epilogue; it is stored to shared memory once the tile buffer is free.
-template <int EPI>
+// (x tiles) x (y tiles) x B grid in a pipeline: while tile t's epilogue runs, tile t + 1's MMAs run (its halo was stored
+// before tile t's wait, into the next of three buffers, and it has the other accumulator) and tile t + 2's halo is on
+// its way into registers. Three buffers, because a slower warp may still read tile t - 1's residual input: one barrier
+// a tile. Each accumulator has its mbarrier, whose phase alternates with its uses.
+// The FP32 residual gradient acc32 belongs to these kernels alone: float4 ((tile 8 + (channel / 4)) 128 + pixel row m),
+// so that a warp's accesses are contiguous (at [pixel][channel] they touched 32 lines each).
+// 4 x 320 x 320, cold, before and after pipeline and layout: hidden layer 31.7 -> 29.3 us, data gradient 59.6 -> 41.0
+// (184 MB: 27 at copy rate), output layer 32.3 -> 19.4 and its data gradient 38.1 -> 25.2 (warp MMAs before).
+template <int EPI, int CIN, int COUT>
 __global__ void __launch_bounds__(kConvTcThreads, 4) conv3x3_tc(const bf16* __restrict__ in, const bf16* __restrict__ w,
                                                             const float* __restrict__ bias, int B, int H, int W,
                                                             bf16* __restrict__ out, bf16* __restrict__ zsave,
-                                                            int* __restrict__ err, float* __restrict__ acc32) {
-  static_assert(EPI == EPI_RELU_RES || EPI == EPI_ACC, "epilogues of the 32 -> 32 layers");
+                                                            int* __restrict__ err, float* __restrict__ f32) {
+  using C = ConvTc<CIN, COUT>;
+  static_assert(EPI == EPI_F32 ? COUT == 8 : COUT == 32, "epilogues");
+  static_assert(EPI != EPI_RELU_RES || CIN == COUT, "residual layers");
   extern __shared__ unsigned char conv_smem_raw[];
   const uint32_t off = tc::smem_addr(conv_smem_raw);
   unsigned char* sm = conv_smem_raw + ((1024u - (off & 1023u)) & 1023u);
-  const uint32_t in_base = tc::smem_addr(sm), w_base = in_base + kConvTcIn;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kConvTcIn + kConvTcW);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  float* bias_s = reinterpret_cast<float*>(sm + kConvTcIn + kConvTcW + 16);
+  const uint32_t in_base = tc::smem_addr(sm), w_base = in_base + kConvTcBufs * C::kIn;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kConvTcBufs * C::kIn + C::kW);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
+  float* bias_s = reinterpret_cast<float*>(bar + 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ntx = (W + kConvTcTW - 1) / kConvTcTW, nty = (H + kConvTcTH - 1) / kConvTcTH;
   const int ntiles = ntx * nty * B;
-  if (tid < CH) bias_s[tid] = bias ? bias[tid] : 0.f;
+  if (tid < COUT) bias_s[tid] = bias ? bias[tid] : 0.f;
   if (tid == 0) {
-    tc::mbar_init(bar, 1);
+    tc::mbar_init(&bar[0], 1);
+    tc::mbar_init(&bar[1], 1);
     tc::fence_mbar_init();
   }
-  if (warp == 0) tc::tmem_alloc(tslot, 32);
-  // weights: item (tap, group, co) at byte ((tap 4 + g) 32 + co) 16
-  for (int i = tid; i < NTAP * 4 * 32; i += kConvTcThreads) {
-    const int co = i & 31, g = (i >> 5) & 3, tap = i >> 7;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(w + ((size_t)tap * CH + co) * CH) + g);
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(w_base + 16 * i), "r"(v.x), "r"(v.y), "r"(v.z),
-                 "r"(v.w)
-                 : "memory");
+  if (warp == 0) tc::tmem_alloc(tslot, C::kCols);
+  // weights: item (tap, group, co) at byte ((tap kGroups + g) kN + co) 16, zero past COUT
+  for (int i = tid; i < NTAP * C::kGroups * C::kN; i += kConvTcThreads) {
+    const int co = i % C::kN, g = (i / C::kN) % C::kGroups, tap = i / (C::kN * C::kGroups);
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (co < COUT) v = __ldg(reinterpret_cast<const uint4*>(w + ((size_t)tap * COUT + co) * CIN) + g);
+    st_shared_v4(w_base + 16 * i, v);
   }
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t tmem = *tslot;
   const int q = warp & 3, h = warp >> 2;
   // the halo of tile t: item i = (pixel, channel group) of 16 bytes, zero outside the image
-  uint4 pre[kConvTcPre];
+  uint4 pre[C::kPre];
   auto fetch = [&](int t) {
     const int bx = t % ntx, by = (t / ntx) % nty, b = t / (ntx * nty);
     const int x0 = bx * kConvTcTW, y0 = by * kConvTcTH;
-    const bf16* inb = in + (size_t)b * H * W * CH;
+    const bf16* inb = in + (size_t)b * H * W * CIN;
 #pragma unroll
-    for (int j = 0; j < kConvTcPre; ++j) {
+    for (int j = 0; j < C::kPre; ++j) {
       const int i = tid + j * kConvTcThreads;
-      const int g = i & 3, pix = i >> 2;
+      const int g = i % C::kGroups, pix = i / C::kGroups;
       const int hy = pix / (kConvTcTW + 2), hx = pix - hy * (kConvTcTW + 2);
       const int gy = y0 + hy - 1, gx = x0 + hx - 1;
       pre[j] = make_uint4(0u, 0u, 0u, 0u);
-      if (i < kConvTcItems && gy >= 0 && gy < H && gx >= 0 && gx < W)
-        pre[j] = __ldg(reinterpret_cast<const uint4*>(inb + ((size_t)gy * W + gx) * CH) + g);
+      if (i < C::kItems && gy >= 0 && gy < H && gx >= 0 && gx < W)
+        pre[j] = __ldg(reinterpret_cast<const uint4*>(inb + ((size_t)gy * W + gx) * CIN) + g);
     }
   };
-  bool ok = true;
-  int it = 0;
-  if (blockIdx.x < ntiles) fetch(blockIdx.x);
-  for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++it) {
-    const int bx = t % ntx, by = (t / ntx) % nty, b = t / (ntx * nty);
-    const int x0 = bx * kConvTcTW, y0 = by * kConvTcTH;
-    // the tile buffer is free (the previous tile's MMAs and epilogue are done)
+  auto stage = [&](uint32_t buf) {
 #pragma unroll
-    for (int j = 0; j < kConvTcPre; ++j) {
+    for (int j = 0; j < C::kPre; ++j) {
       const int i = tid + j * kConvTcThreads;
-      if (i < kConvTcItems)
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(in_base + (i & 3) * kConvTcGroup + 16 * (i >> 2)),
-                     "r"(pre[j].x), "r"(pre[j].y), "r"(pre[j].z), "r"(pre[j].w)
-                     : "memory");
+      if (i < C::kItems) st_shared_v4(buf + (i % C::kGroups) * C::kGroup + 16 * (i / C::kGroups), pre[j]);
     }
     tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    // (the test hook withholds block 0's first tile: no MMAs and no commit, so the wait below runs out)
-    if (tid == 0 && !(it == 0 && blockIdx.x == 0 && tc::g_drop_arrival)) {
-      const uint32_t idesc = tc::idesc_bf16(128, CH);
-      for (int tap = 0; tap < NTAP; ++tap) {
-        const uint32_t a0 = in_base + 16 * ((tap / 3) * (kConvTcTW + 2) + tap % 3);
-        for (int k = 0; k < 2; ++k)  // channel groups 2k, 2k + 1
-          tc::mma_bf16(tmem, tc::desc_interleave(a0 + 2 * k * kConvTcGroup, kConvTcGroup, 16 * (kConvTcTW + 2)),
-                       tc::desc_interleave(w_base + (tap * 4 + 2 * k) * 512, 512, 128), idesc, (tap | k) ? 1u : 0u);
-      }
-      tc::mma_commit(bar);
+  };
+  uint32_t tmem = 0;
+  auto issue = [&](uint32_t buf, int s) {  // the MMAs of the CTA's tile number s, by one thread
+    const uint32_t idesc = tc::idesc_bf16(128, C::kN), d = tmem + C::kN * (s & 1);
+    for (int tap = 0; tap < NTAP; ++tap) {
+      const uint32_t a0 = buf + 16 * ((tap / 3) * (kConvTcTW + 2) + tap % 3);
+      for (int k = 0; k < C::kGroups / 2; ++k)  // channel groups 2k, 2k + 1
+        tc::mma_bf16(d, tc::desc_interleave(a0 + 2 * k * C::kGroup, C::kGroup, 16 * (kConvTcTW + 2)),
+                     tc::desc_interleave(w_base + (tap * C::kGroups + 2 * k) * (16 * C::kN), 16 * C::kN, 128), idesc,
+                     (tap | k) ? 1u : 0u);
     }
-    if (t + (int)gridDim.x < ntiles) fetch(t + gridDim.x);
-    const int m = 32 * q + lane, gy = y0 + (m >> 3), gx = x0 + (m & 7);  // row m = pixel (m % 8, m / 8)
+    tc::mma_commit(&bar[s & 1]);
+  };
+  const int step = gridDim.x;
+  uint32_t cur = in_base, nxt = in_base + C::kIn;  // buffers of this tile and the next
+  if ((int)blockIdx.x < ntiles) {
+    fetch(blockIdx.x);
+    stage(cur);
+  }
+  if ((int)blockIdx.x + step < ntiles) fetch(blockIdx.x + step);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  tmem = *tslot;
+  // (the test hook withholds block 0's first tile: no MMAs and no commit, so the wait below runs out)
+  if (tid == 0 && (int)blockIdx.x < ntiles && !(blockIdx.x == 0 && tc::g_drop_arrival)) issue(cur, 0);
+  bool ok = true;
+  int it = 0;
+  for (int t = blockIdx.x; t < ntiles; t += step, ++it) {
+    if (t + step < ntiles) {  // tile it + 1 of the grid: its MMAs run while this tile's epilogue does
+      stage(nxt);
+      tc::fence_before_sync();
+      ok = __syncthreads_and(ok);
+      tc::fence_after_sync();
+      if (!ok) break;  // an earlier wait gave up; this tile's MMAs may be in flight (waited for below)
+      if (tid == 0) issue(nxt, it + 1);
+      if (t + 2 * step < ntiles) fetch(t + 2 * step);
+    }
+    const int bx = t % ntx, by = (t / ntx) % nty, b = t / (ntx * nty);
+    const int m = 32 * q + lane, gy = by * kConvTcTH + (m >> 3), gx = bx * kConvTcTW + (m & 7);  // row m = pixel (m % 8, m / 8)
     const bool inside = gy < H && gx < W;
     const size_t pix = ((size_t)b * H + gy) * W + gx;
-    float4 acc_in[4];  // the accumulated gradient and the layer below's pre-activation, loaded while the MMAs run
+    // the accumulated gradient and the layer below's pre-activation, loaded while the MMAs run
+    float4* ap = reinterpret_cast<float4*>(f32) + ((size_t)t * 8 + 4 * h) * 128 + m;
+    float4 acc_in[4];
     uint4 zin[2];
-    if constexpr (EPI == EPI_ACC) {
+    if constexpr (EPI == EPI_ACC || EPI == EPI_F32_BF16) {
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4) acc_in[q4] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (inside) {
         const uint4* zp = reinterpret_cast<const uint4*>(zsave + pix * CH + 16 * h);
         zin[0] = zp[0];
         zin[1] = zp[1];
-        const float4* ap = reinterpret_cast<const float4*>(acc32 + pix * CH + 16 * h);
+        if (EPI == EPI_ACC)
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) acc_in[q4] = ap[q4];
+          for (int q4 = 0; q4 < 4; ++q4) acc_in[q4] = ap[128 * q4];
       }
     }
-    ok = tc::mbar_wait(bar, it & 1);  // every thread waits each phase in turn
+    const bool done = tc::mbar_wait(&bar[it & 1], (it >> 1) & 1);  // every thread waits each phase in turn
     // after a give-up, wait once more (bounded) for MMAs still in flight before the tile buffer, the
     // accumulator and finally the tensor memory are released
-    if (!ok) tc::mbar_wait(bar, it & 1);
+    if (!done) tc::mbar_wait(&bar[it & 1], (it >> 1) & 1);
+    ok = ok && done;
     tc::fence_after_sync();
     float v[16];
-    tc::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + 16 * h, v);
+    tc::tmem_ld16(tmem + C::kN * (it & 1) + ((uint32_t)(32 * q) << 16) + (C::kN == 32 ? 16 * h : 0), v);
     if (ok && inside) {
-      uint32_t o[8], zz[8], res[8];
-      float bs[16];
-      if constexpr (EPI == EPI_RELU_RES) {
+      if constexpr (EPI == EPI_F32) {  // channels 4 h .. 4 h + 3
+        float4 y;
+        y.x = (h ? v[4] : v[0]) + bias_s[4 * h];
+        y.y = (h ? v[5] : v[1]) + bias_s[4 * h + 1];
+        y.z = (h ? v[6] : v[2]) + bias_s[4 * h + 2];
+        y.w = (h ? v[7] : v[3]) + bias_s[4 * h + 3];
+        reinterpret_cast<float4*>(f32 + pix * 8)[h] = y;
+      } else if constexpr (EPI == EPI_RELU_RES) {
+        uint32_t o[8], zz[8], res[8];
+        float bs[16];
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           uint32_t r[4];
@@ -210,152 +241,58 @@ __global__ void __launch_bounds__(kConvTcThreads, 4) conv3x3_tc(const bf16* __re
 #pragma unroll
           for (int e = 0; e < 4; ++e) bs[4 * q4 + e] = __uint_as_float(r[e]);
         }
-      }
-      if constexpr (EPI == EPI_RELU_RES) {  // the residual input: this pixel's channels 16 h .. 16 h + 15 in the tile
-        const uint32_t hp = in_base + 16 * (((m >> 3) + 1) * (kConvTcTW + 2) + (m & 7) + 1);
-        ld_shared_v4(hp + 2 * h * kConvTcGroup, *reinterpret_cast<uint32_t(*)[4]>(&res[0]));
-        ld_shared_v4(hp + (2 * h + 1) * kConvTcGroup, *reinterpret_cast<uint32_t(*)[4]>(&res[4]));
-      }
+        // the residual input: this pixel's channels 16 h .. 16 h + 15 in the tile
+        const uint32_t hp = cur + 16 * (((m >> 3) + 1) * (kConvTcTW + 2) + (m & 7) + 1);
+        ld_shared_v4(hp + 2 * h * C::kGroup, *reinterpret_cast<uint32_t(*)[4]>(&res[0]));
+        ld_shared_v4(hp + (2 * h + 1) * C::kGroup, *reinterpret_cast<uint32_t(*)[4]>(&res[4]));
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {  // output channels 16 h + 2 j, + 1
-        float z0 = v[2 * j], z1 = v[2 * j + 1];
-        if constexpr (EPI == EPI_RELU_RES) {
-          z0 += bs[2 * j];
-          z1 += bs[2 * j + 1];
-        }
-        if constexpr (EPI == EPI_ACC) {
-          o[j] = pack_bf16(z0, z1);
-        } else {
+        for (int j = 0; j < 8; ++j) {  // output channels 16 h + 2 j, + 1
+          const float z0 = v[2 * j] + bs[2 * j], z1 = v[2 * j + 1] + bs[2 * j + 1];
           zz[j] = pack_bf16(z0, z1);
           const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162*>(&res[j]);
           o[j] = pack_bf16(__bfloat162float(hv.x) + fmaxf(z0, 0.f), __bfloat162float(hv.y) + fmaxf(z1, 0.f));
         }
-      }
-      if constexpr (EPI == EPI_ACC) {
-        float4* ap = reinterpret_cast<float4*>(acc32 + pix * CH + 16 * h);
+        uint4* op = reinterpret_cast<uint4*>(out + pix * CH + 16 * h);
+        op[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        op[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        if (zsave) {  // (inference keeps no pre-activations)
+          uint4* zp = reinterpret_cast<uint4*>(zsave + pix * CH + 16 * h);
+          zp[0] = make_uint4(zz[0], zz[1], zz[2], zz[3]);
+          zp[1] = make_uint4(zz[4], zz[5], zz[6], zz[7]);
+        }
+      } else {
+        uint32_t o[8];
+        const uint32_t zi[8] = {zin[0].x, zin[0].y, zin[0].z, zin[0].w, zin[1].x, zin[1].y, zin[1].z, zin[1].w};
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           float4 a = acc_in[q4];
-          const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&o[2 * q4]);
-          const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&o[2 * q4 + 1]);
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(v[4 * q4], v[4 * q4 + 1]);
+          const __nv_bfloat162 hi = __floats2bfloat162_rn(v[4 * q4 + 2], v[4 * q4 + 3]);
           a.x += __bfloat162float(lo.x);
           a.y += __bfloat162float(lo.y);
           a.z += __bfloat162float(hi.x);
           a.w += __bfloat162float(hi.y);
-          ap[q4] = a;
-          // ReLU's derivative on the rounded gradient (z > 0: positive, not zero, as BF16 bits)
-          const uint32_t z01 = q4 == 0 ? zin[0].x : q4 == 1 ? zin[0].z : q4 == 2 ? zin[1].x : zin[1].z;
-          const uint32_t z23 = q4 == 0 ? zin[0].y : q4 == 1 ? zin[0].w : q4 == 2 ? zin[1].y : zin[1].w;
-          o[2 * q4] = relu_mask(pack_bf16(a.x, a.y), z01);
-          o[2 * q4 + 1] = relu_mask(pack_bf16(a.z, a.w), z23);
+          ap[128 * q4] = a;
+          // ReLU's derivative on the rounded gradient
+          o[2 * q4] = relu_mask(pack_bf16(a.x, a.y), zi[2 * q4]);
+          o[2 * q4 + 1] = relu_mask(pack_bf16(a.z, a.w), zi[2 * q4 + 1]);
         }
         uint4* gp = reinterpret_cast<uint4*>(out + pix * CH + 16 * h);
         gp[0] = make_uint4(o[0], o[1], o[2], o[3]);
         gp[1] = make_uint4(o[4], o[5], o[6], o[7]);
-      } else {
-        uint4* op = reinterpret_cast<uint4*>(out + pix * CH + 16 * h);
-        op[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        op[1] = make_uint4(o[4], o[5], o[6], o[7]);
-      }
-      if (EPI == EPI_RELU_RES && zsave) {  // (inference keeps no pre-activations)
-        uint4* zp = reinterpret_cast<uint4*>(zsave + pix * CH + 16 * h);
-        zp[0] = make_uint4(zz[0], zz[1], zz[2], zz[3]);
-        zp[1] = make_uint4(zz[4], zz[5], zz[6], zz[7]);
       }
     }
-    ok = __syncthreads_and(ok);  // the tile buffer and the accumulator are free for the next tile
+    cur = nxt;
+    nxt = nxt + C::kIn < w_base ? nxt + C::kIn : in_base;
   }
-  if (!ok && tid == 0) atomicExch(err, 0x2000);
+  // left early: the tile whose turn it was has its MMAs in flight (bounded)
+  if (!ok && (int)blockIdx.x + it * step < ntiles) tc::mbar_wait(&bar[it & 1], (it >> 1) & 1);
+  if (!ok) atomicExch(err, 0x2000);
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem, 32);
-  }
-}
-
-// 3 x 3 convolution as an implicit GEMM on warp-level MMAs, for the layers tcgen05 does not take (N = 8
-// output channels; the 16-channel padded output gradient): in: [B][H][W][CIN] BF16; w: [9][COUT][CIN] BF16;
-// bias: [COUT] FP32 (may be null); FP32 output. Each block computes a 16 x 8 pixel tile; warp w owns tile
-// row w (16 pixels = one M tile).
-template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(32 * TH) conv3x3_mma(const bf16* __restrict__ in, const bf16* __restrict__ w,
-                                                       const float* __restrict__ bias, int H, int W,
-                                                       float* __restrict__ out32, const bf16* __restrict__ z,
-                                                       bf16* __restrict__ out) {
-  static_assert(CIN % 16 == 0 && COUT % 8 == 0, "channel counts");
-  static_assert(EPI == EPI_F32 || EPI == EPI_F32_BF16, "epilogues of the 32 -> 8 layer and the first data gradient");
-  constexpr int PS = CIN + 4;       // smem pixel stride (bf16): spreads the fragment loads over all banks
-  constexpr int WS = CIN + 8;       // smem weight row stride (bf16)
-  __shared__ __align__(16) bf16 s_in[(TH + 2) * (TW + 2) * PS];
-  __shared__ __align__(16) bf16 s_w[NTAP * COUT * WS];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int gid = lane >> 2, tig = lane & 3;
-  const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH, b = blockIdx.z;
-  const bf16* inb = in + (size_t)b * H * W * CIN;
-  // stage weights and the input tile with a one-pixel halo (zero outside the image), 4-byte granules
-  for (int i = tid; i < NTAP * COUT * (CIN / 2); i += blockDim.x) {
-    const int row = i / (CIN / 2), c2 = i - row * (CIN / 2);
-    reinterpret_cast<uint32_t*>(s_w + row * WS)[c2] = reinterpret_cast<const uint32_t*>(w + (size_t)row * CIN)[c2];
-  }
-  for (int i = tid; i < (TH + 2) * (TW + 2) * (CIN / 2); i += blockDim.x) {
-    const int pix = i / (CIN / 2), c2 = i - pix * (CIN / 2);
-    const int ty = pix / (TW + 2), tx = pix - ty * (TW + 2);
-    const int gy = y0 - 1 + ty, gx = x0 - 1 + tx;
-    uint32_t v = 0;
-    if (gy >= 0 && gy < H && gx >= 0 && gx < W)
-      v = reinterpret_cast<const uint32_t*>(inb + ((size_t)gy * W + gx) * CIN)[c2];
-    reinterpret_cast<uint32_t*>(s_in + pix * PS)[c2] = v;
-  }
-  __syncthreads();
-  float acc[COUT / 8][4];
-#pragma unroll
-  for (int n = 0; n < COUT / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-#pragma unroll
-  for (int tap = 0; tap < NTAP; ++tap) {
-    const int ky = tap / 3, kx = tap % 3;
-    const bf16* arow0 = s_in + ((warp + ky) * (TW + 2) + gid + kx) * PS;  // pixel gid of this warp's row
-    const bf16* arow1 = arow0 + 8 * PS;                                    // pixel gid + 8
-#pragma unroll
-    for (int kk = 0; kk < CIN / 16; ++kk) {
-      uint32_t a[4];
-      const int c = kk * 16 + tig * 2;
-      a[0] = *reinterpret_cast<const uint32_t*>(arow0 + c);
-      a[1] = *reinterpret_cast<const uint32_t*>(arow1 + c);
-      a[2] = *reinterpret_cast<const uint32_t*>(arow0 + c + 8);
-      a[3] = *reinterpret_cast<const uint32_t*>(arow1 + c + 8);
-#pragma unroll
-      for (int n = 0; n < COUT / 8; ++n) {
-        const bf16* brow = s_w + (tap * COUT + n * 8 + gid) * WS + c;
-        mma16816(acc[n], a, *reinterpret_cast<const uint32_t*>(brow), *reinterpret_cast<const uint32_t*>(brow + 8));
-      }
-    }
-  }
-  // epilogue: rows gid and gid + 8 of the M tile are pixels x0 + gid (+ 8) of image row y0 + warp
-  const int gy = y0 + warp;
-  if (gy >= H) return;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int gx = x0 + gid + 8 * half;
-    if (gx >= W) continue;
-    const size_t pix = ((size_t)b * H + gy) * W + gx;
-#pragma unroll
-    for (int n = 0; n < COUT / 8; ++n) {
-      const int co = n * 8 + tig * 2;
-      float z0 = acc[n][2 * half], z1 = acc[n][2 * half + 1];
-      if (bias) {
-        z0 += bias[co];
-        z1 += bias[co + 1];
-      }
-      if constexpr (EPI == EPI_F32) {
-        *reinterpret_cast<float2*>(out32 + pix * COUT + co) = c2(z0, z1);
-      } else {
-        *reinterpret_cast<float2*>(out32 + pix * COUT + co) =
-            c2(__bfloat162float(__float2bfloat16(z0)), __bfloat162float(__float2bfloat16(z1)));
-        *reinterpret_cast<uint32_t*>(out + pix * COUT + co) =
-            relu_mask(pack_bf16(z0, z1), *reinterpret_cast<const uint32_t*>(z + pix * COUT + co));
-      }
-    }
+    tc::tmem_dealloc(tmem, C::kCols);
   }
 }
 
@@ -395,16 +332,13 @@ __global__ void __launch_bounds__(kWgThreads, kWgPerSm) wgrad_tc(const bf16* __r
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ntx = (W + TW - 1) / TW, nty = (H + TH - 1) / TH;
   const int ntiles = ntx * nty * B;
-  auto st16 = [](uint32_t addr, uint4 v) {
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-  };
   if (tid == 0) {
     tc::mbar_init(bar, 1);
     tc::fence_mbar_init();
   }
   if (warp == 0) tc::tmem_alloc(tslot, kCols);
   for (int i = tid; i < (TH + 2) * TW; i += kWgThreads)  // the ones: BF16 1 in the group's first channel
-    st16(a_base + 12 * kWgGroupA + 16 * i, make_uint4(0x3F80u, 0u, 0u, 0u));
+    st_shared_v4(a_base + 12 * kWgGroupA + 16 * i, make_uint4(0x3F80u, 0u, 0u, 0u));
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -443,13 +377,13 @@ __global__ void __launch_bounds__(kWgThreads, kWgPerSm) wgrad_tc(const bf16* __r
 #pragma unroll
         for (int kx = 0; kx < 3; ++kx) {
           const int p = col - kx;
-          if (p >= 0 && p < TW) st16(a_base + (kx * 4 + cg) * kWgGroupA + 16 * (hy * TW + p), px[j]);
+          if (p >= 0 && p < TW) st_shared_v4(a_base + (kx * 4 + cg) * kWgGroupA + 16 * (hy * TW + p), px[j]);
         }
     }
 #pragma unroll
     for (int j = 0; j < kPreD; ++j) {
       const int i = tid + j * kWgThreads, cg = i % (NC / 8), p = i / (NC / 8);
-      if (i < kD) st16(b_base + cg * kWgGroupB + 16 * p, pd[j]);
+      if (i < kD) st_shared_v4(b_base + cg * kWgGroupB + 16 * p, pd[j]);
     }
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -561,9 +495,12 @@ __global__ void flip_transpose(const bf16* __restrict__ w, LayerOffsets o, bf16*
 __global__ void __launch_bounds__(256) conv_in_fwd(const float* __restrict__ x, const float* __restrict__ w,
                                                    const float* __restrict__ bias, int B, int H, int W,
                                                    bf16* __restrict__ out, bf16* __restrict__ zsave) {
-  __shared__ float2 sw[NTAP * CH];
-  __shared__ float sb[CH];
-  for (int i = threadIdx.x; i < NTAP * CH; i += blockDim.x) sw[i] = reinterpret_cast<const float2*>(w)[i];
+  __shared__ __align__(16) float sw[NTAP * CH * 2];  // [tap][channel pair][input channel][channel of the pair]
+  __shared__ __align__(8) float sb[CH];
+  for (int i = threadIdx.x; i < NTAP * CH * 2; i += blockDim.x) {
+    const int ci = i & 1, co = (i >> 1) % CH, tap = i / (2 * CH);
+    sw[((tap * (CH / 2) + (co >> 1)) * 2 + ci) * 2 + (co & 1)] = w[i];
+  }
   if (threadIdx.x < CH) sb[threadIdx.x] = bias[threadIdx.x];
   __syncthreads();
   const size_t n = (size_t)B * H * W;
@@ -581,20 +518,15 @@ __global__ void __launch_bounds__(256) conv_in_fwd(const float* __restrict__ x, 
       uint32_t zz[4], oo[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        float z[2];
+        float2 z = *reinterpret_cast<const float2*>(&sb[c8 + 2 * q]);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int co = c8 + 2 * q + j;
-          float s = sb[co];
-#pragma unroll
-          for (int tap = 0; tap < NTAP; ++tap) {
-            const float2 wt = sw[tap * CH + co];
-            s += wt.x * in[tap].x + wt.y * in[tap].y;
-          }
-          z[j] = s;
+        for (int tap = 0; tap < NTAP; ++tap) {
+          const float4 wt = *reinterpret_cast<const float4*>(&sw[(tap * (CH / 2) + c8 / 2 + q) * 4]);
+          const float2 v = __fmul2_rn(c2(wt.z, wt.w), c2(in[tap].y, in[tap].y));
+          z = __fadd2_rn(z, __ffma2_rn(c2(wt.x, wt.y), c2(in[tap].x, in[tap].x), v));
         }
-        zz[q] = pack_bf16(z[0], z[1]);
-        oo[q] = pack_bf16(fmaxf(z[0], 0.f), fmaxf(z[1], 0.f));
+        zz[q] = pack_bf16(z.x, z.y);
+        oo[q] = pack_bf16(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f));
       }
       if (zsave) reinterpret_cast<uint4*>(zsave + p * CH)[c8 / 8] = make_uint4(zz[0], zz[1], zz[2], zz[3]);
       reinterpret_cast<uint4*>(out + p * CH)[c8 / 8] = make_uint4(oo[0], oo[1], oo[2], oo[3]);
@@ -605,14 +537,14 @@ __global__ void __launch_bounds__(256) conv_in_fwd(const float* __restrict__ x, 
 // Weight and bias gradients of the 2 -> 32 input layer, stage 1: lane = output channel co; a warp takes row segments
 // of kSeg pixels and keeps the 3 x 3 window of the two input channels in registers, so that a pixel costs three
 // (broadcast) window loads, one 64-byte load of g[p][0..31] and the 19 accumulations (all nine taps loaded and bounds-
-// checked per pixel: 134 us for 4 x 320 x 320, now 54). The warps' sums are added in warp order in shared memory:
+// checked per pixel: 134 us for 4 x 320 x 320, now 47). The warps' sums are added in warp order in shared memory:
 // partial[b][(tap CH + co) 2 + ci] = sum x[p + d(tap)][ci] g[p][co], partial[b][NTAP CH 2 + co] = sum g[p][co].
 // sum_partials adds the blocks in a fixed order.
 constexpr int kConvInPartial = NTAP * CH * 2 + CH;
-constexpr int kPartialBlocksPerSm = 8;  // at most so many blocks per SM of the partial-sum kernels
+constexpr int kPartialBlocksPerSm = 4;  // what is resident
 constexpr int kConvInWarps = 8;
 constexpr int kSeg = 32;
-__global__ void __launch_bounds__(32 * kConvInWarps) conv_in_wgrad_partial(const float* __restrict__ x,
+__global__ void __launch_bounds__(32 * kConvInWarps, kPartialBlocksPerSm) conv_in_wgrad_partial(const float* __restrict__ x,
                                                                            const bf16* __restrict__ g, int B, int H,
                                                                            int W, float* __restrict__ partial) {
   __shared__ float sh[kConvInWarps][2 * NTAP + 1][CH];
@@ -648,8 +580,7 @@ __global__ void __launch_bounds__(32 * kConvInWarps) conv_in_wgrad_partial(const
       sb += gv;
 #pragma unroll
       for (int t = 0; t < NTAP; ++t) {
-        acc[t].x += win[t / 3][t % 3].x * gv;
-        acc[t].y += win[t / 3][t % 3].y * gv;
+        acc[t] = __ffma2_rn(win[t / 3][t % 3], c2(gv, gv), acc[t]);
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -861,8 +792,16 @@ class WarmStartCnn {
       all.resize(at, 0.f);
     }
     upload_params(all.data());
-    for (auto fn : {conv3x3_tc<EPI_ACC>, conv3x3_tc<EPI_RELU_RES>}) {
-      PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kConvTcSmem));
+    const struct {
+      decltype(&conv3x3_tc<EPI_ACC, CH, CH>) fn;
+      int smem;
+    } convs[] = {{conv3x3_tc<EPI_RELU_RES, CH, CH>, (int)ConvTc<CH, CH>::kSmem},
+                 {conv3x3_tc<EPI_ACC, CH, CH>, (int)ConvTc<CH, CH>::kSmem},
+                 {conv3x3_tc<EPI_F32, CH, 8>, (int)ConvTc<CH, 8>::kSmem},
+                 {conv3x3_tc<EPI_F32_BF16, 16, CH>, (int)ConvTc<16, CH>::kSmem}};
+    for (auto& c : convs) {
+      auto fn = c.fn;
+      PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, c.smem));
       // all of the unified L1 / shared storage as shared memory, so that several CTAs fit on an SM
       PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     }
@@ -882,12 +821,12 @@ class WarmStartCnn {
     PDT_CUDA_CHECK(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     PDT_CUDA_CHECK(cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev));
     PDT_CUDA_CHECK(cudaDeviceGetAttribute(&thr_sm, cudaDevAttrMaxThreadsPerMultiProcessor, dev));
-    for (auto fn : {conv3x3_tc<EPI_ACC>, conv3x3_tc<EPI_RELU_RES>}) {
+    for (auto& c : convs) {
       cudaFuncAttributes fa{};
-      PDT_CUDA_CHECK(cudaFuncGetAttributes(&fa, fn));
+      PDT_CUDA_CHECK(cudaFuncGetAttributes(&fa, c.fn));
       const int warp_regs = ((fa.numRegs * 32 + 255) / 256) * 256;
       const int by_regs = regs_sm / (warp_regs * (kConvTcThreads / 32));
-      const int by_smem = smem_sm / ((int)kConvTcSmem + (int)fa.sharedSizeBytes + smem_rsv);
+      const int by_smem = smem_sm / (c.smem + (int)fa.sharedSizeBytes + smem_rsv);
       const int by_thr = thr_sm / kConvTcThreads;
       conv_tc_per_sm_ = std::min({conv_tc_per_sm_, by_regs, by_smem, by_thr});
     }
@@ -925,17 +864,16 @@ class WarmStartCnn {
                                                keep ? z_[0].as<bf16>() : nullptr);
     PDT_LAUNCH_CHECK();
     count_launch(2);
-    const dim3 grid((W + TW - 1) / TW, (H + TH - 1) / TH, B);
     const int tgrid = conv_tc_grid(B, H, W);
     for (int l = 1; l <= 6; ++l) {
-      conv3x3_tc<EPI_RELU_RES><<<tgrid, kConvTcThreads, kConvTcSmem, st>>>(h_[l - 1].as<bf16>(), W_[l].wb, B_[l].w, B, H, W,
-                                                                         h_[l].as<bf16>(), keep ? z_[l].as<bf16>() : nullptr,
-                                                                         err_.as<int>(), nullptr);
+      conv3x3_tc<EPI_RELU_RES, CH, CH><<<tgrid, kConvTcThreads, ConvTc<CH, CH>::kSmem, st>>>(
+          h_[l - 1].as<bf16>(), W_[l].wb, B_[l].w, B, H, W, h_[l].as<bf16>(), keep ? z_[l].as<bf16>() : nullptr,
+          err_.as<int>(), nullptr);
       PDT_LAUNCH_CHECK();
       count_launch();
     }
-    conv3x3_mma<CH, 8, EPI_F32><<<grid, 32 * TH, 0, st>>>(h_[6].as<bf16>(), W_[7].wb, B_[7].w, H, W, o_.as<float>(),
-                                                          nullptr, nullptr);
+    conv3x3_tc<EPI_F32, CH, 8><<<tgrid, kConvTcThreads, ConvTc<CH, 8>::kSmem, st>>>(
+        h_[6].as<bf16>(), W_[7].wb, B_[7].w, B, H, W, nullptr, nullptr, err_.as<int>(), o_.as<float>());
     PDT_LAUNCH_CHECK();
     count_launch();
   }
@@ -952,23 +890,22 @@ class WarmStartCnn {
     flip_transpose<<<dim3(36, 7), 256, 0, st>>>(pb_.as<bf16>(), at, wt_.as<bf16>());
     auto wt = [&](int l) { return wt_.as<bf16>() + (size_t)(l - 1) * NTAP * CH * CH; };
     PDT_LAUNCH_CHECK();
-    const dim3 grid((W + TW - 1) / TW, (H + TH - 1) / TH, B);
     const int tgrid = conv_tc_grid(B, H, W);
     // conv_out: dW, db, and dh6 = conv(go, W7') (8 -> 32 channels, padded to 16 input channels), with which the
     // residual stream's FP32 gradient starts as G = dh6 (the BF16 rounding of the convolution's output)
     wgrad(8, h_[6].as<bf16>(), go_.as<bf16>(), B, H, W, W_[7].g, st);
     bf16* gz = gz_[0].as<bf16>();  // dz = G * relu'(z_l) of the layer at hand; the next layer's goes to the other buffer
     bf16* gn = gz_[1].as<bf16>();
-    conv3x3_mma<16, CH, EPI_F32_BF16><<<grid, 32 * TH, 0, st>>>(go_.as<bf16>(), wt(7), nullptr, H, W, gacc_.as<float>(),
-                                                                z_[6].as<bf16>(), gz);
+    conv3x3_tc<EPI_F32_BF16, 16, CH><<<tgrid, kConvTcThreads, ConvTc<16, CH>::kSmem, st>>>(
+        go_.as<bf16>(), wt(7), nullptr, B, H, W, gz, z_[6].as<bf16>(), err_.as<int>(), gacc_.as<float>());
     PDT_LAUNCH_CHECK();
-    count_launch(3);  // mse_loss, flip_transpose, conv3x3_mma
+    count_launch(3);  // mse_loss, flip_transpose, conv3x3_tc
     for (int l = 6; l >= 1; --l) {
       // h_l = h_{l-1} + relu(z_l), z_l = conv_l(h_{l-1}):  dh_{l-1} = G + conv_l^T(dz), added into the FP32 residual
       // gradient in the convolution's epilogue, which also masks it for the layer below
       wgrad(CH, h_[l - 1].as<bf16>(), gz, B, H, W, W_[l].g, st);
-      conv3x3_tc<EPI_ACC><<<tgrid, kConvTcThreads, kConvTcSmem, st>>>(gz, wt(l), nullptr, B, H, W, gn, z_[l - 1].as<bf16>(),
-                                                                    err_.as<int>(), gacc_.as<float>());
+      conv3x3_tc<EPI_ACC, CH, CH><<<tgrid, kConvTcThreads, ConvTc<CH, CH>::kSmem, st>>>(
+          gz, wt(l), nullptr, B, H, W, gn, z_[l - 1].as<bf16>(), err_.as<int>(), gacc_.as<float>());
       PDT_LAUNCH_CHECK();
       count_launch();
       std::swap(gz, gn);
@@ -1063,7 +1000,8 @@ class WarmStartCnn {
     o_.ensure(npix * 8 * sizeof(float));
     go_.ensure(npix * 16 * sizeof(bf16));
     for (auto& g : gz_) g.ensure(npix * CH * sizeof(bf16));
-    gacc_.ensure(npix * CH * sizeof(float));
+    const size_t tiles = (size_t)B * ((W + kConvTcTW - 1) / kConvTcTW) * ((H + kConvTcTH - 1) / kConvTcTH);
+    gacc_.ensure(tiles * kConvTcTW * kConvTcTH * CH * sizeof(float));
     wt_.ensure((size_t)7 * NTAP * CH * CH * sizeof(bf16));
     B_n_ = B;
     H_n_ = H;
@@ -1091,7 +1029,7 @@ class WarmStartCnn {
   DevBuf x_, h_[7], z_[7], o_, go_, gz_[2], gacc_, wt_, wpart_, part_, t_, sc_, err_, bpart_;
 
   int sms_ = 1;
-  int conv_tc_per_sm_ = 8;  // resident conv3x3_tc CTAs per SM (each holds 32 TMEM columns: 8 x 32 <= 512)
+  int conv_tc_per_sm_ = 8;  // resident conv3x3_tc CTAs per SM (each holds 64 TMEM columns: 8 x 64 <= 512)
   int B_n_ = 0, H_n_ = 0, W_n_ = 0;
   long step_ = 0;
 };
