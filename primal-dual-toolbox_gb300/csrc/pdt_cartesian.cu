@@ -30,6 +30,7 @@
 #include <mutex>
 #include <sstream>
 
+#include "pdt_cart_rows.h"
 #include "pdt_cart_tiles.h"
 #include "pdt_device.cuh"
 #include "pdt_fftplan.h"
@@ -311,7 +312,9 @@ class CartesianOp : public OpImpl, public SolverHooks {
     check_device_errors();
     std::ostringstream os;
     os << "W=" << dev_.W << " H=" << dev_.Hf << " C=" << dev_.C << " sampled_columns=" << dev_.ns;
-    if (tune_.tcf)
+    if (tune_.rf)
+      os << " rows_fwd=register_fft";
+    else if (tune_.tcf)
       os << " rows_fwd=tensor_dft(tf32x3,k_split=" << tune_.ks << ",stages=" << tc_fwd_stages() << ")";
     else if (frow_.ok())
       os << " rows_fwd=lane_fft(" << frow_.M << "x" << frow_.L << ",warps=" << kWpbChoices[tune_.wf]
@@ -321,7 +324,9 @@ class CartesianOp : public OpImpl, public SolverHooks {
          << ")";
     else
       os << " rows_fwd=stockham";
-    if (tune_.tca)
+    if (tune_.ra)
+      os << " rows_adj=register_fft(cluster)";
+    else if (tune_.tca)
       os << " rows_adj=tensor_dft(tf32x3,n_ranges=" << (2 * dev_.W + tc_adj_nb(tune_.nr) - 1) / tc_adj_nb(tune_.nr)
          << ",row_tiles=" << tc_adj_tiles() << "x" << tc_adj_yb() << "rows,stages=" << tc_adj_stages(tc_adj_nb(tune_.nr))
          << ",coil_sum_on_chip)";
@@ -342,7 +347,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
     if (gram_.len.n)
       os << " solver=line_gram(" << gram_.len.P << "x" << gram_.len.Q << (gram_.len.n == dev_.W ? "" : ",padded") << ",coil_sums="
          << gram_.groups << ")";
-    if (frow_.ok())  // what a batched solve runs (tca(), tcf(), groups_run())
+    if (frow_.ok() && !tune_.ra)  // what a batched solve runs (tca(), tcf(), groups_run())
       os << " in_batch=lane_fft_rows(batch_adj_groups=" << std::min(G_, batch_groups())
          << (tune_.cluster ? ",cluster" : ",partials") << ")";
     return os.str();
@@ -379,7 +384,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
   }
   int groups() override {
     prepare();
-    if (tca()) return 1;                         // the tensor-core adjoint rows sum the coils on chip
+    if (tca() || ra()) return 1;                 // these adjoint rows sum the coils on chip
     return (frow_.ok() && tune_.cluster) ? 1 : groups_run();  // a cluster reduces its coil groups on chip
   }
   long long group_stride() override { return (long long)dev_.Hi * dev_.W; }
@@ -409,12 +414,17 @@ class CartesianOp : public OpImpl, public SolverHooks {
       return;
     }
     float2* t = scratch_.as<float2>();
-    launch_rows_fwd(ubar, t, tick, st);
+    if (rf())
+      launch_row_fft_fwd(row_fft_, ubar, t, tick, nullptr, 0, st);
+    else
+      launch_rows_fwd(ubar, t, tick, st);
     if (mk) mk->mark("cart_rows_fwd", st);
     launch_cols(COL_SOLVE, t, t, r, fc, nullptr, nullptr, sigma, lambda, st);
     if (mk) mk->mark("cart_cols_prox", st);
     if (tca())
       launch_tc_rows_adj(t, khr, st, dual);  // the coil sum on chip: one K^H r plane
+    else if (ra())
+      launch_row_fft_adj(row_fft_, t, khr, st);
     else
       launch_rows_adj(t, khr, groups_run(), st);
     if (mk) mk->mark("cart_rows_adj", st);
@@ -427,10 +437,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
     }
     float2* t = scratch_.as<float2>();
     launch_cols(COL_ADJ_COMPACT, nullptr, t, nullptr, fc, nullptr, nullptr, 0.f, 0.f, st);
-    if (tca() && !exact_rows)
-      launch_tc_rows_adj(t, img, st);
-    else
-      launch_rows_adj(t, img, 1, st);
+    launch_rows_image(t, img, st, exact_rows);
   }
 
  protected:
@@ -455,10 +462,14 @@ class CartesianOp : public OpImpl, public SolverHooks {
   }
   void execute_forward(const float2* src, float2* dst, cudaStream_t st) override {
     prepare();
-    launch_fill_zero(dst, sizeof(float2) * (size_t)dev_.C * dev_.Hf * dev_.W, st);
+    const size_t nk = (size_t)dev_.C * dev_.Hf * dev_.W;
+    if (!rf()) launch_fill_zero(dst, sizeof(float2) * nk, st);
     if (dev_.ns == 0) return;
     float2* t = scratch_.as<float2>();
-    launch_rows_fwd(src, t, nullptr, st);
+    if (rf())
+      launch_row_fft_fwd(row_fft_, src, t, nullptr, dst, nk, st);  // and dst <- 0
+    else
+      launch_rows_fwd(src, t, nullptr, st);
     launch_cols(COL_FWD_DENSE, t, nullptr, nullptr, nullptr, nullptr, dst, 0.f, 0.f, st);
   }
   void execute_adjoint(const float2* src, float2* dst, cudaStream_t st) override {
@@ -469,16 +480,14 @@ class CartesianOp : public OpImpl, public SolverHooks {
     }
     float2* t = scratch_.as<float2>();
     launch_cols(COL_ADJ_DENSE, nullptr, t, nullptr, nullptr, src, nullptr, 0.f, 0.f, st);
-    if (tca())
-      launch_tc_rows_adj(t, dst, st);
-    else
-      launch_rows_adj(t, dst, 1, st);
+    launch_rows_image(t, dst, st, false);
   }
   void invalidate() override { prepared_ = false; }
 
  private:
   // Launch configuration of the lane-FFT kernels, chosen by the autotuner in prepare().
   struct Tune {
+    int rf = 0, ra = 0;          // 1: register-transform forward / adjoint rows
     int wf = 2, wc = 2, wa = 2;  // warps-per-block index (kWpbChoices) of rows_fwd, cols, rows_adj
     bool cluster = false;        // coil groups of a row block reduced in a cluster (else partial images)
     int tcf = 0, tca = 0;        // 1: tensor-core DFT rows (forward / adjoint) instead of the FFT kernels
@@ -576,6 +585,12 @@ class CartesianOp : public OpImpl, public SolverHooks {
     return cap;
   }
   int groups_run() const { return concurrent_ ? std::min(G_, batch_groups()) : G_; }
+  // The register-transform rows (pdt_cart_rows.h), alone and in a batch, in place of the tuned lane-FFT or tensor-core
+  // rows where they were faster (a forward and an adjoint one after the other, lane-FFT or tensor-core rows against
+  // these, 15 coils 640 x 368: 82 us against 68; 12 coils 256 x 256 with a 2-D mask: 77 against 39), and always against
+  // the generic rows (4 coils 120 x 112: 48 against 37).
+  bool rf() const { return tune_.rf != 0; }
+  bool ra() const { return tune_.ra != 0; }
   bool tcf() const { return tune_.tcf && !(concurrent_ && frow_.ok()); }
 
   void launch_rows_fwd(const float2* ubar, float2* t1, int* tick, cudaStream_t st) {
@@ -621,6 +636,15 @@ class CartesianOp : public OpImpl, public SolverHooks {
     static const char* env = std::getenv("PDT_ROWS_ADJ_STAGED");
     const bool want = (env && *env) ? std::atoi(env) != 0 : tune_.sst != 0;
     return want && fast_rows_adj_smem(dev_, k, wpb, true) <= (size_t)g_max_smem;
+  }
+  // K^H as one image; `exact`: in FP32 (the tensor-core rows carry 22 bits).
+  void launch_rows_image(const float2* t, float2* img, cudaStream_t st, bool exact) {
+    if (tca() && !exact)
+      launch_tc_rows_adj(t, img, st);
+    else if (row_fft_ok_ && !pinned_)
+      launch_row_fft_adj(row_fft_, t, img, st);
+    else
+      launch_rows_adj(t, img, 1, st);
   }
   // K^H: G coil-group partial images (or, with a cluster, one reduced image) into out.
   void launch_rows_adj(const float2* t2, float2* out, int G, cudaStream_t st) {
@@ -808,6 +832,20 @@ class CartesianOp : public OpImpl, public SolverHooks {
     const int row_blocks = (d.Hi + d.RB - 1) / d.RB;
     G_ = std::max(1, std::min(C, (2 * g_num_sms + row_blocks - 1) / row_blocks));
     dev_ = d;
+    row_fft_ok_ = row_fft_ok(W, d.ns, d.sens != nullptr, g_max_smem);
+    row_fft_.W = W;
+    row_fft_.Hi = d.Hi;
+    row_fft_.C = C;
+    row_fft_.ns = d.ns;
+    row_fft_.mx = d.mxW % W;
+    row_fft_.ox = d.oxW;
+    row_fft_.sens = d.sens ? d.sens + (size_t)d.y0 * W : nullptr;
+    row_fft_.coil_stride = (size_t)Hf * W;
+    row_fft_.tw = d.twW;
+    row_fft_.fs2s = d.fslot2s;
+    row_fft_.as2s = d.slot2s;
+    pinned_ = false;
+    tune_.rf = tune_.ra = row_fft_ok_;  // where nothing is tuned: against the generic rows
     autotune();
     dev_ = d;
     prepare_gram(mask, col_x);
@@ -912,6 +950,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
       }
     };
     const uint64_t launches0 = g_launches.load();
+    tune_.rf = tune_.ra = 0;
     Tune best = tune_;
     float bt = 1e30f, ba = 1e30f;  // best forward / adjoint row times so far
     if (frow_.ok()) {
@@ -954,6 +993,10 @@ class CartesianOp : public OpImpl, public SolverHooks {
       }
       tune_.tcf = 0;
     }
+    if (row_fft_ok_) {
+      const float ms = time([&] { launch_row_fft_fwd(row_fft_, ub.as<float2>(), t, nullptr, nullptr, 0, st); });
+      if (ms < bt) bt = ms, best.rf = 1, best.tcf = 0;
+    }
     if (fcol_.ok()) {
       float bc = 1e30f;
       for (int w = 0; w < 3; ++w) {
@@ -977,6 +1020,11 @@ class CartesianOp : public OpImpl, public SolverHooks {
         const float ms = time([&] { launch_tc_rows_adj(t, kh.as<float2>(), st); });
         if (ms < pair) pair = ms, best.tca = 1, best.nr = nr;
       }
+      ba = pair;
+    }
+    if (row_fft_ok_) {
+      const float ms = time([&] { launch_row_fft_adj(row_fft_, t, kh.as<float2>(), st); });
+      if (ms < ba) ba = ms, best.ra = 1, best.tca = 0;
     }
     if (const int e = take_tc_error()) {
       std::fprintf(stderr, "pdt: tensor-core row kernels reported error %d while tuning; using the FFT rows\n", e);
@@ -998,6 +1046,8 @@ class CartesianOp : public OpImpl, public SolverHooks {
   bool pinned_tune() {
     const char* env = std::getenv("PDT_CARTESIAN_TUNE");
     if (!env || !*env) return false;
+    pinned_ = true;
+    tune_.rf = tune_.ra = 0;
     int v[9];
     const int n = std::sscanf(env, "%d,%d,%d,%d,%d,%d,%d,%d,%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6],
                               &v[7], &v[8]);
@@ -1031,6 +1081,8 @@ class CartesianOp : public OpImpl, public SolverHooks {
   }
 
   bool prepared_ = false;
+  RowFft row_fft_;
+  bool row_fft_ok_ = false, pinned_ = false;
   Tune tune_;
   CartDev dev_{};
   FastRowKernels frow_;
