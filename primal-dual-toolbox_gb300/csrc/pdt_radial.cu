@@ -223,7 +223,7 @@ __global__ void rad_transpose(RadDev d, const float2* __restrict__ in, float2* _
 // Gridding as a gather: H[gy][gx][c] = sum_j s[j][c] wx[gx - gx0_j] wy[gy - gy0_j] over the samples j whose
 // footprint covers the cell (lists built at set-up, entries in sample order). One launch, two kinds of block:
 // the first n_heavy blocks take a cell near k = 0 (more than kHeavy entries) each, thread (slot, coil) summing
-// every slots-th entry and the slots added in order; the others give each (cell, coil) a thread that walks the
+// every slots-th entry and the slots added pairwise; the others give each (cell, coil) a thread that walks the
 // cell's list in order, four entries at a time so that many loads are in flight. A warp's loads of s are runs of C
 // values (a thread per cell and all coils, as before, touched 32 runs a load: 20 us instead of 6 for 12 coils on 384^2).
 template <int V>
@@ -244,11 +244,13 @@ __global__ void __launch_bounds__(kRT) rad_grid(RadDev d, const float2* __restri
         for (int e = beg + slot; e < end; e += slots) acc += s[(size_t)d.cell_idx[e] * C + c] * d.cell_w[e];
       }
       part[threadIdx.x] = acc;
-      __syncthreads();
-      if (slot == 0 && c < C) {
-        for (int q = 1; q < slots; ++q) acc += part[q * cw + c0];
-        H[(size_t)cell * C + c] = acc;
+      // pairwise: one coil has 256 slots, and adding these one after the other doubled the adjoint's rounding error
+      for (int n = slots, h; n > 1; n = h) {
+        h = (n + 1) / 2;
+        __syncthreads();
+        if (slot + h < n) part[threadIdx.x] += part[threadIdx.x + h * cw];
       }
+      if (slot == 0 && c < C) H[(size_t)cell * C + c] = part[threadIdx.x];
       __syncthreads();
     }
     return;
