@@ -184,6 +184,19 @@ def _phase_bytes_case(C, Hf, W, ns, G, roos):
     }
 
 
+def _line_gram_bytes(N, C, sums):
+    """Algorithmic bytes per launch of a line-sampled solve's two kernels (N image pixels, C coils, `sums`
+    coil-group sums of K^H K U): the row operator reads U and the maps and writes the sums; the image kernel reads
+    u, v(2), p(2), q(3), K^H f, U with its compensation and the sums and writes u, v, p, q and U again."""
+    return {"mri_gram_rows": 8 * N * (1 + C + sums), "mri_image_tgv": 8 * N * (8 + 1 + 2 + sums + 8 + 2)}
+
+
+def _coil_sums(tuning):
+    """Coil-group sums of a solver on the row operator ('... solver=line_gram(23x16,coil_sums=1)'), or None."""
+    m = re.search(r"solver=line_gram\([^)]*coil_sums=(\d+)\)", tuning)
+    return int(m.group(1)) if m else None
+
+
 def _phase_bytes(ns, G, fused_dual=False):
     """Algorithmic bytes per launch of each kernel phase (each logical array read or written once). With
     the dual update run by extra blocks of the adjoint-rows launch (fused_dual), that launch moves both."""
@@ -268,9 +281,10 @@ def run_ours(args):
 
     # per-kernel timing (CUDA events on the launching stream) for the roofline of the dominant kernel
     phases = opt.profile(iters=50, stream=stream)
+    sums = _coil_sums(op.tuning())
     G = _khr_planes(op.tuning())
-    fused_dual = "solver_dual=adjoint_launch" in op.tuning()
-    bytes_per = _phase_bytes(ns, G, fused_dual)
+    fused_dual = sums is None and "solver_dual=adjoint_launch" in op.tuning()
+    bytes_per = _phase_bytes(ns, G, fused_dual) if sums is None else _line_gram_bytes(H // 2 * W, C, sums)
     per_iter_ms = sum(phases.values())
     dom = max(phases, key=phases.get)
     hbm, src = _peaks()
@@ -286,6 +300,13 @@ def run_ours(args):
     phase_info = {k: {"ms": round(v, 5), "GB/s": round(bytes_per.get(k, 0) / (v / 1e3) / 1e9, 1)}
                   for k, v in phases.items()}
     tuning = op.tuning()
+    if "mri_gram_rows" in phases:
+        # the row operator's working set stays in L2: it is bound by FP32 arithmetic, a transform pair of each row and
+        # coil and the two products with the maps; the peak is 152 SMs x 128 lanes x 2 x 2.07 GHz (nominal)
+        flop = C * (H // 2) * (2 * 5 * W * np.log2(W) + 16 * W)
+        ach = flop / (phases["mri_gram_rows"] / 1e3) / 1e12
+        phase_info["mri_gram_rows"]["fp32"] = {"bound": "fp32", "achieved": round(ach, 2), "peak": 80.5, "unit": "TFLOP/s",
+                                               "frac": round(ach / 80.5, 4), "flop": int(flop), "peak_source": "nominal"}
     if "rows_adj=tensor_dft" in tuning and "cart_rows_adj" in phases:
         # tensor-core DFT adjoint rows: one real GEMM pass is 2 (C Hi) (2 W) (2 ns) flops; the TF32 hi/lo
         # split executes three; the TF32 peak is half the measured dense BF16 rate (the tensor cores'
@@ -571,8 +592,6 @@ def _khr_planes(tuning):
     """K^H r planes the adjoint row phase writes and the image step reads: 1 when the coil groups are
     reduced in a thread-block cluster, else one partial image per coil group (from the operator's
     tuning report, e.g. '... rows_adj=register_fft(warps=4,coil_groups=6,partials) ...')."""
-    import re
-
     m = re.search(r"coil_groups=(\d+)(,cluster|,partials)?", tuning)
     if not m:
         return 1
@@ -684,10 +703,15 @@ def run_batched(pdt, torch, n_cases, iters, steps, warmup):
         opt.setNoisyData(case["rawdata"])
         ns = int((case["mask"] != 0).any(axis=0).sum())
         tuning = op.tuning()
-        G, lane_in_batch = _batch_khr_planes(tuning)
-        adj = "tensor_dft" if "rows_adj=tensor_dft" in tuning and not lane_in_batch else "lane_fft"
+        sums = _coil_sums(tuning)
+        if sums is not None:
+            adj = "line_gram"
+            nbytes += sum(_line_gram_bytes(spec["H"] * spec["W"], spec["C"], sums).values())
+        else:
+            G, lane_in_batch = _batch_khr_planes(tuning)
+            adj = re.search(r"rows_adj=(\w+)", tuning).group(1) if not lane_in_batch else "lane_fft"
+            nbytes += sum(_phase_bytes_case(spec["C"], spec["H"], spec["W"], ns, G, False).values())
         adj_rows[adj] = adj_rows.get(adj, 0) + 1
-        nbytes += sum(_phase_bytes_case(spec["C"], spec["H"], spec["W"], ns, G, False).values())
         pix += spec["H"] * spec["W"]
         opts.append(opt)
         ops.append(op)
@@ -924,21 +948,21 @@ def run_cufft(pdt, torch, case, dev, op, phases, reps=50):
         "cufft_fft2_only_ms": timed(lambda: torch.fft.fft2(k, norm="ortho")),
         "cufft_iteration_operator_ms": timed(lambda: ref.prox_step(u, r, dev["rawdata"], 0.125, 1.0)),
     }
-    ours_iter = sum(v for n, v in phases.items() if n.startswith("cart_"))
+    ours_iter = sum(v for n, v in phases.items() if n.startswith(("cart_", "mri_gram")))
     out = {n: round(v, 4) for n, v in t.items()}
     out["ours_iteration_operator_ms"] = round(ours_iter, 4)
     out["speedup_forward"] = round(t["cufft_forward_ms"] / t["ours_forward_ms"], 2)
     out["speedup_adjoint"] = round(t["cufft_adjoint_ms"] / t["ours_adjoint_ms"], 2)
     out["speedup_iteration_operator"] = round(t["cufft_iteration_operator_ms"] / ours_iter, 2)
     out["note"] = ("ours forward writes the full masked k-space and adjoint reads it (as the reference API); "
-                   "the iteration operator touches only sampled columns")
+                   "the iteration operator touches only sampled columns, or for whole sampled lines is K^H K row by row")
     return out
 
 
 def run_ncu_case(args):
     """The workload's kernels for an ncu capture: operator set-up, autotuning and graph capture run first,
     then one solve of --ncu-iters iterations runs between cudaProfilerStart and cudaProfilerStop, so
-    `ncu --profile-from-start off` sees exactly those launches (5 kernels per Cartesian iteration, 9 per
+    `ncu --profile-from-start off` sees exactly those launches (2 kernels per line-sampled Cartesian iteration, 7 per
     radial iteration)."""
     import torch
 

@@ -843,8 +843,8 @@ class OptImpl {
   // iteration's dual update, whose first one runs here. The operator part is the round with the k-space dual, or for a
   // line mask the row operator (pdt_gram.h): then b = K^H f and z0 = K^H r_0 are formed here and the k-space dual
   // follows from U after the iterations. u, v, U alternate between two copies with the iteration (the free halves of
-  // the slab), p and q with the state's parity. An error of b acts like one of the data in every iteration, so its
-  // rows are transformed in FP32 (with the tensor-core rows u was 1.5e-6 off after 1001 iterations instead of 4e-7).
+  // the slab), p and q with the state's parity. An error of b acts in every iteration, also where the mask does not see
+  // it: its rows are transformed in FP32, and from kPairMinIters iterations on it is a pair of FP32 images.
   void plan_image(Plan& pl, const GramRows* gram, SolverHooks* hk, int G, bool r_zero, float tau, float sigma,
                   float lambda, float k, float c, float d, cudaStream_t st) {
     const size_t N = (size_t)W_ * H_, plane = plane_bytes();
@@ -854,18 +854,21 @@ class OptImpl {
     const bool is_tgv = kind_ != PDT_OPT_TV_OP;
     int* header = alpha_.as<int>();
     const float4* table = reinterpret_cast<const float4*>(alpha_.as<char>() + kAlphaHeader);
-    float2 *U = nullptr, *b = nullptr, *z0 = nullptr, *part = khr_.as<float2>();
-    if (row_op) {  // two copies of {U, compensation}, b, z0, partial sums
-      const size_t bytes = (6 + (size_t)groups) * plane;
+    float2 *U = nullptr, *b = nullptr, *b_lo = nullptr, *z0 = nullptr, *part = khr_.as<float2>();
+    if (row_op) {  // two copies of {U, compensation}, b and its remainder, z0, partial sums
+      const size_t bytes = (7 + (size_t)groups) * plane;
       if (gram_.bytes != bytes) {
         gram_.ensure(bytes);
         ++version_;
       }
       U = gram_.as<float2>();
       b = U + 4 * N;
-      z0 = b + N;
+      z0 = b + 2 * N;
       part = z0 + N;
-      hk->adjoint_compact(fc_.as<float2>(), b, st, true);
+      if (n >= kPairMinIters && hk->adjoint_pair(fc_.as<float2>(), b, b + N, st))
+        b_lo = b + N;
+      else
+        hk->adjoint_compact(fc_.as<float2>(), b, st, true);
       if (!r_zero) hk->adjoint_compact(r_.as<float2>(), z0, st, true);
       launch_gram_start(W_, H_, static_cast<const float2*>(field(F_UB, p0)), k, U, st);
     }
@@ -892,6 +895,7 @@ class OptImpl {
         g.U = U + 2 * N * par;
         g.Unext = U + 2 * N * (par ^ 1);
         g.b = b;
+        g.b_lo = b_lo;
         g.z0 = r_zero ? nullptr : z0;
       }
       g.part = part;
@@ -924,7 +928,7 @@ class OptImpl {
     pl.key = graph_key({(uintptr_t)img_.p, (uintptr_t)gram_.p, (uintptr_t)khr_.p, (uintptr_t)r_.p, (uintptr_t)fc_.p,
                         (uintptr_t)alpha_.p, (uintptr_t)alpha_.bytes, (uintptr_t)op_.get(), (uintptr_t)op_->generation(),
                         (uintptr_t)W_, (uintptr_t)H_, (uintptr_t)groups, (uintptr_t)p0, (uintptr_t)is_tgv,
-                        (uintptr_t)r_zero, (uintptr_t)row_op, fbits(lambda), fbits(tau), fbits(sigma),
+                        (uintptr_t)r_zero, (uintptr_t)row_op, (uintptr_t)b_lo, fbits(lambda), fbits(tau), fbits(sigma),
                         (uintptr_t)version_, (uintptr_t)1});
   }
 
@@ -979,6 +983,7 @@ class OptImpl {
   static constexpr int kGraphIters = 20;
   static constexpr size_t kAlphaHeader = 64;
   static constexpr unsigned kGramMinIters = 8;
+  static constexpr int kPairMinIters = 256;  // see plan_image() and pdt_cart_pair.cuh
 
   pdt_opt_kind kind_;
   bool cplx_;

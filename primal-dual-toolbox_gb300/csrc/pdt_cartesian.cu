@@ -260,6 +260,7 @@ void query_device() {
 }  // namespace pdt
 
 #include "pdt_cart_fast.cuh"
+#include "pdt_cart_pair.cuh"
 #include "pdt_cart_tc.cuh"
 
 namespace pdt {
@@ -428,6 +429,33 @@ class CartesianOp : public OpImpl, public SolverHooks {
     else
       launch_rows_adj(t, khr, groups_run(), st);
     if (mk) mk->mark("cart_rows_adj", st);
+  }
+  bool adjoint_pair(const float2* fc, float2* img, float2* lo, cudaStream_t st) override {
+    prepare();
+    int nq = std::min(4, dev_.C);
+    while (nq > 1 && pair_rows_smem(dev_.W, nq) > 100 * 1024) --nq;
+    const size_t cs = pair_cols_smem(dev_.Hf), rs = pair_rows_smem(dev_.W, nq), smem = std::max(cs, rs);
+    if (dev_.ns == 0 || smem > (size_t)g_max_smem) return false;
+    if (!pair_built_) {
+      std::vector<float4> h, w;
+      pair_twiddles(dev_.Hf, h);
+      pair_twiddles(dev_.W, w);
+      h.insert(h.end(), w.begin(), w.end());
+      pair_tab_.ensure(h.size() * sizeof(float4));
+      PDT_CUDA_CHECK(cudaMemcpy(pair_tab_.p, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
+      pair_t_.ensure((size_t)dev_.C * dev_.ns * dev_.Hi * sizeof(float4));
+      PDT_CUDA_CHECK(cudaFuncSetAttribute(pair_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
+      PDT_CUDA_CHECK(cudaFuncSetAttribute(pair_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
+      pair_built_ = true;
+    }
+    const float4* tw = pair_tab_.as<float4>();
+    const float2 scale = pair_of(1.0 / std::sqrt((double)dev_.W * dev_.Hf));
+    pair_cols<<<dim3(dev_.ns, dev_.C), kPairThreads, cs, st>>>(dev_, tw, fc, pair_t_.as<float4>());
+    PDT_LAUNCH_CHECK();
+    pair_rows<<<dev_.Hi, kPairThreads, rs, st>>>(dev_, tw + dev_.Hf, pair_t_.as<float4>(), nq, scale, img, lo);
+    PDT_LAUNCH_CHECK();
+    count_launch(2);
+    return true;
   }
   void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool exact_rows) override {
     prepare();
@@ -844,7 +872,7 @@ class CartesianOp : public OpImpl, public SolverHooks {
     row_fft_.tw = d.twW;
     row_fft_.fs2s = d.fslot2s;
     row_fft_.as2s = d.slot2s;
-    pinned_ = false;
+    pinned_ = pair_built_ = false;
     tune_.rf = tune_.ra = row_fft_ok_;  // where nothing is tuned: against the generic rows
     autotune();
     dev_ = d;
@@ -1083,6 +1111,8 @@ class CartesianOp : public OpImpl, public SolverHooks {
   bool prepared_ = false;
   RowFft row_fft_;
   bool row_fft_ok_ = false, pinned_ = false;
+  DevBuf pair_tab_, pair_t_;  // adjoint_pair(): twiddles of Hf and W, columns of [c][s][yi]
+  bool pair_built_ = false;
   Tune tune_;
   CartDev dev_{};
   FastRowKernels frow_;

@@ -188,12 +188,16 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   const bool in = tid < (GX + 1) * (GY + 1) && x < W && y < H;
   const bool own = in && lx < GX && ly < GY;
   const size_t idx = in ? (size_t)y * W + x : 0;
-  float2 ou = c2(0.f, 0.f), kf = ou, ovx = ou, ovy = ou, Uo = ou, Ue = ou;
+  float2 ou = c2(0.f, 0.f), kf = ou, ke = ou, ovx = ou, ovy = ou, Uo = ou, Ue = ou;
   if (in) {
     ou = ld(s.src.u, idx);
     if constexpr (ROWS) {
-      kf = row.z * __ldcg(s.b + idx);
-      if (s.z0) kf = kf - row.w * __ldcg(s.z0 + idx);
+      // c K^H f as the rounded product and the rest: both it and K^H K U are far larger than their difference
+      const float2 b = __ldcg(s.b + idx);
+      kf = c2(__fmul_rn(row.z, b.x), __fmul_rn(row.z, b.y));
+      ke = c2(__fmaf_rn(row.z, b.x, -kf.x), __fmaf_rn(row.z, b.y, -kf.y));
+      if (s.b_lo) ke = ke + row.z * __ldcg(s.b_lo + idx);
+      if (s.z0) ke = ke - row.w * __ldcg(s.z0 + idx);
     }
     if constexpr (TGV) {
       ovx = ld(s.src.vx, idx);
@@ -254,7 +258,7 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   if (in) {
     float2 kh = s.part[idx];
     for (int g = 1; g < s.groups; ++g) kh += s.part[idx + (size_t)g * W * H];
-    if constexpr (ROWS) kh = kh - kf;
+    if constexpr (ROWS) kh = (kh - kf) - ke;
     const float2 un = ou + s.tau * (dp - kh);
     s_ub[ly][lx] = 2.0f * un - ou;
     finite = finite && isfinite(un.x) && isfinite(un.y);

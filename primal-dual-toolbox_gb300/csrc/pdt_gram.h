@@ -60,6 +60,7 @@ struct GramImage {
   const float2* part;    // `groups` partial sums of K^H K U, W x H each
   int groups;
   const float2* b;       // K^H f
+  const float2* b_lo;    // what b as FP32 leaves of it, or null
   const float2* z0;      // K^H r_0, or null when r_0 = 0
   const float4* table;   // per iteration {alpha0, alpha1, c, d}
   int* header;           // [1] table length, [2] non-finite flag, [4], [5] iteration counters (see par)

@@ -59,6 +59,9 @@ struct SolverHooks {
   // `exact_rows`: with row transforms whose error is that of FP32 rounding also where another kernel (TF32
   // triples, about 1e-6 relative) is faster.
   virtual void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool exact_rows = false) = 0;
+  // The same as a sum of two FP32 images, accurate to FP64 rounding of the data; false (and nothing done) where the
+  // operator has no such adjoint.
+  virtual bool adjoint_pair(const float2* /*fc*/, float2* /*img*/, float2* /*lo*/, cudaStream_t /*st*/) { return false; }
 };
 
 class OpImpl {

@@ -76,3 +76,28 @@ def test_other_masks_keep_the_three_passes(pdt):
     op.setCoilSens(np.ones((2, 20, 24), np.complex64))
     op.setMask(mask)
     assert "solver=line_gram" not in op.tuning()
+
+
+# rows and columns whose transforms have radices 2 to 5, a prime of their own and a padded row; 256 iterations are the
+# first number with K^H f as a pair of FP32 images
+@pytest.mark.parametrize("C,H,W,roos,n", [(8, 96, 92, False, 1001), (3, 58, 31, False, 256), (5, 80, 48, True, 400)])
+def test_long_solves_keep_the_k_space_duals_accuracy(pdt, oracle, C, H, W, roos, n):
+    from primaldualtoolbox import synthetic
+
+    case = synthetic.cartesian_case(C=C, H=H, W=W, roos=roos, seed=0)
+    op = (pdt.mri.MriCartesianRemoveROOSOperator if roos else pdt.mri.MriCartesianOperator)()
+    op.setCoilSens(case["sens"])
+    op.setMask(case["mask"])
+    assert "solver=line_gram" in op.tuning()
+    o = pdt.mri.TgvMriOptimizer_2c3c()
+    prm = o.getParameters()
+    prm.max_iter, prm.reduction, prm.alpha1 = n - 1, 0.01, case["alpha1"]
+    prm.alpha0 = 2 * prm.alpha1
+    o.setOperator(op)
+    o.setNoisyData(case["rawdata"])
+    o.solve()
+    ref = oracle.op_solve("cartesian_roos" if roos else "cartesian", case["sens"], case["mask"], case["rawdata"], "tgv_mri",
+                          alpha0=float(prm.alpha0), alpha1=float(prm.alpha1), reduction=0.01, max_iter=n - 1, prec=64)
+    # a NumPy model of the first case's 1001 iterations in FP32 ends 3.0e-7 off with the k-space dual, 3.3e-7 with the
+    # row operator and K^H f in 64 bits, 1.2e-6 with K^H f in FP32; twice the middle one
+    assert rel_l2(o.getResult(), ref) <= 6.6e-7
