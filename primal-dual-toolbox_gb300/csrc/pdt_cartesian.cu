@@ -1,5 +1,6 @@
 // pdt_cartesian.cu -- Cartesian multi-coil MRI operators (plain and readout-oversampling removal) and
-// the single-coil sampling operator, as three shared-memory FFT phases.
+// the single-coil sampling operator, as three FFT phases (rows, sampled columns, rows back); masks of whole lines also
+// have the row operator of pdt_gram.h.
 //
 // Reference: MriCartesianOperator / MriCartesianRemoveROOSOperator (mricartesianoperator.cu:27-414)
 // and MriSamplingOperator (mrisamplingoperator.cu:58-88):

@@ -7,10 +7,10 @@
 //   h_{l+1} = h_l + relu(conv_l(h_l)), l = 1..6    32 -> 32
 //   o  = conv_out(h7)                              32 -> 8 (6 used)
 //   u  = u0 + s (o0 + i o1),  v = s (o2 + i o3, o4 + i o5)
-// Eight convolutions in all. The 32-channel convolutions run as implicit GEMMs on the tensor cores
-// (mma.sync m16n8k16, BF16 in, FP32 accumulate): pixels are the M dimension, output channels N, and
-// (tap, input channel) K. The data gradient is the same kernel with flipped taps and transposed channels;
-// the weight gradient is a second implicit GEMM with pixels as K, reduced over blocks in block order.
+// Eight convolutions in all. All but the first run as implicit GEMMs on the tensor cores (tcgen05, BF16 in, FP32
+// accumulate): pixels are the M dimension, output channels N, and (tap, input channel) K. The data gradient is the
+// same kernel with flipped taps and transposed channels; the weight gradient is a second implicit GEMM with pixels
+// as K, reduced over blocks in block order.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -434,9 +434,10 @@ __global__ void __launch_bounds__(kWgThreads, kWgPerSm) wgrad_tc(const bf16* __r
   }
 }
 
-// grad[i] = sum over the blocks b of partial[b][i], in a fixed order: a block takes 32 outputs, each of its 16 warps
-// a range of b in order, and the warps' sums are added in order.
-constexpr int kWgSumWarps = 16;
+// grad[i] = sum over the blocks b of partial[b][i], in a fixed order: a block takes 32 outputs, each of its 32 warps
+// a range of b in order, and the warps' sums are added in order. Bound by the loads' latency (a training step of
+// 4 x 320 x 320, seven of these: 922 us with 32 warps, 940 with 16 or 8).
+constexpr int kWgSumWarps = 32;
 __global__ void __launch_bounds__(32 * kWgSumWarps) wgrad_sum(const float* __restrict__ partial, int nblocks, int n,
                                                               float* __restrict__ grad) {
   __shared__ float sh[kWgSumWarps][32];
@@ -984,7 +985,7 @@ class WarmStartCnn {
     PDT_LAUNCH_CHECK();
     PDT_CUDA_CHECK(cudaDeviceSynchronize());
   }
-  // persistent tensor-core convolutions: three CTAs per SM (66 KB of shared memory each), at most one tile each
+  // persistent tensor-core convolutions: what is resident (four CTAs per SM by registers), at most one tile each
   int conv_tc_grid(int B, int H, int W) const {
     const long long tiles = (long long)((W + kConvTcTW - 1) / kConvTcTW) * ((H + kConvTcTH - 1) / kConvTcTH) * B;
     return (int)std::min<long long>(tiles, (long long)conv_tc_per_sm_ * sms_);

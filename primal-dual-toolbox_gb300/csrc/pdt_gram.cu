@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
 // row kernel starts, and nothing the row kernel reads is written here, so the divergences, the v update and
 // the next q run before the programmatic wait (L2 loads: this SM may hold older lines). Bound by the latency
 // of its load phases: four blocks an SM (48 registers, some spilled) make one wave of the 480 blocks of a
-// 320 x 368 image and 17.6 us an iteration with the row kernel; three blocks 21.2, two 19.7.
+// 320 x 368 image and 17.6 us an iteration with the row kernel; three blocks 21.2, two 19.7 (before the product's
+// rounding error and the pair's remainder, which add 0.5).
 // ------------------------------------------------------------------------------------------------
 constexpr int GX = 32, GY = 8, GT = 320;  // (GX + 1) (GY + 1) = 297 primal pixels, one a thread
 
