@@ -749,9 +749,21 @@ class OptImpl {
       PDT_CUDA_CHECK(cudaMemsetAsync(r_.p, 0, r_.bytes, st));
       r_reset_ = false;
     }
-    // A line mask: an iteration is two launches (pdt_gram.h). Its set-up and the k-space dual at its end are
-    // two adjoints and one forward, which fewer than kGramMinIters iterations do not pay back.
-    const GramRows* gram = params_.max_iter + 1 >= kGramMinIters ? hk->line_gram() : nullptr;
+    // step sizes (tgvmrioptimizer.cu:132-134; *withop.cu: tau = sigma = 1/8)
+    float tau = kind_ == PDT_OPT_TGV_MRI ? 1.0f / 16.0f : 1.0f / 8.0f;
+    float sigma = 1.0f / 8.0f;
+    if (step_tau_ > 0.f) tau = step_tau_;  // pdt_opt_set_steps (no reference counterpart)
+    if (step_sigma_ > 0.f) sigma = step_sigma_;
+    const float lambda = kind_ == PDT_OPT_TGV_MRI ? 1.0f : (float)params_.lambda;
+    const unsigned K = params_.max_iter;
+    const int n = (int)K + 1;
+    const float gk = sigma / (1.0f + sigma * lambda);
+    double gc_last = 0;  // the last iteration's c
+    for (int k = 0; k < n && gc_last <= kGramMaxC; ++k) gc_last += (double)gk * (1.0 - (double)lambda * gc_last);
+    // A line mask: an iteration is two launches (pdt_gram.h).
+    const GramRows* gram = n >= kGramMinIters && gc_last <= kGramMaxC ? hk->line_gram() : nullptr;
+    if (gram && n < kGramMinItersLarge && (size_t)gram->C * gram->W * gram->H >= kGramLarge) gram = nullptr;
+    if (gram && !reserve_row_op(*gram, hk)) gram = nullptr;
     const int G = hk->groups();
     const long long gstride = hk->group_stride();
     const size_t khr_bytes = (size_t)G * gstride * sizeof(float2);
@@ -759,20 +771,11 @@ class OptImpl {
       khr_.ensure(khr_bytes);
       ++version_;
     }
-    // step sizes (tgvmrioptimizer.cu:132-134; *withop.cu: tau = sigma = 1/8)
-    float tau = kind_ == PDT_OPT_TGV_MRI ? 1.0f / 16.0f : 1.0f / 8.0f;
-    float sigma = 1.0f / 8.0f;
-    if (step_tau_ > 0.f) tau = step_tau_;  // pdt_opt_set_steps (no reference counterpart)
-    if (step_sigma_ > 0.f) sigma = step_sigma_;
-    const float lambda = kind_ == PDT_OPT_TGV_MRI ? 1.0f : (float)params_.lambda;
     // alpha table for every iteration (tgvmrioptimizer.cu:144-155 in real_type)
-    const unsigned K = params_.max_iter;
-    const int n = (int)K + 1;
     const bool fused = !gram && hk->can_fuse_dual(W_, H_);
     const int ld = fused ? 2 : 4;  // {alpha0, alpha1} or {alpha0, alpha1, c, d}, c and d as in pdt_gram.h
     std::vector<float> tab(ld * (size_t)n);
     double gc = 0, gd = 1;
-    const float gk = sigma / (1.0f + sigma * lambda);
     for (unsigned k = 0; k <= K; ++k) {
       float a0 = (float)params_.alpha0, a1 = (float)params_.alpha1;
       if (kind_ == PDT_OPT_TGV_MRI) alpha_at(k, a0, a1);
@@ -841,10 +844,9 @@ class OptImpl {
 
   // Iterations of an operator part and one image kernel (launch_gram_image): the primal update, then the next
   // iteration's dual update, whose first one runs here. The operator part is the round with the k-space dual, or for a
-  // line mask the row operator (pdt_gram.h): then b = K^H f and z0 = K^H r_0 are formed here and the k-space dual
-  // follows from U after the iterations. u, v, U alternate between two copies with the iteration (the free halves of
-  // the slab), p and q with the state's parity. An error of b acts in every iteration, also where the mask does not see
-  // it: its rows are transformed in FP32, and from kPairMinIters iterations on it is a pair of FP32 images.
+  // line mask the row operator (pdt_gram.h): then w, h and z0 = K^H r_0 are formed here and the k-space dual
+  // follows from D after the iterations. u, v, D alternate between two copies with the iteration (the free halves of
+  // the slab), p and q with the state's parity.
   void plan_image(Plan& pl, const GramRows* gram, SolverHooks* hk, int G, bool r_zero, float tau, float sigma,
                   float lambda, float k, float c, float d, cudaStream_t st) {
     const size_t N = (size_t)W_ * H_, plane = plane_bytes();
@@ -854,23 +856,18 @@ class OptImpl {
     const bool is_tgv = kind_ != PDT_OPT_TV_OP;
     int* header = alpha_.as<int>();
     const float4* table = reinterpret_cast<const float4*>(alpha_.as<char>() + kAlphaHeader);
-    float2 *U = nullptr, *b = nullptr, *b_lo = nullptr, *z0 = nullptr, *part = khr_.as<float2>();
-    if (row_op) {  // two copies of {U, compensation}, b and its remainder, z0, partial sums
-      const size_t bytes = (7 + (size_t)groups) * plane;
-      if (gram_.bytes != bytes) {
-        gram_.ensure(bytes);
-        ++version_;
-      }
-      U = gram_.as<float2>();
-      b = U + 4 * N;
-      z0 = b + 2 * N;
+    float2 *D = nullptr, *w = nullptr, *h = nullptr, *z0 = nullptr, *part = khr_.as<float2>();
+    if (row_op) {  // reserve_row_op()'s planes
+      D = gram_.as<float2>();
+      w = D + 4 * N;
+      h = w + N;
+      z0 = h + N;
       part = z0 + N;
-      if (n >= kPairMinIters && hk->adjoint_pair(fc_.as<float2>(), b, b + N, st))
-        b_lo = b + N;
-      else
-        hk->adjoint_compact(fc_.as<float2>(), b, st, true);
+      hk->adjoint_compact(fc_.as<float2>(), w, st, true);
+      launch_gram_rows(rows, w, part, st);
+      launch_gram_start(W_, H_, part, groups, static_cast<const float2*>(field(F_UB, p0)), k, w, D, part + groups * N, st);
+      hk->adjoint_residual(w, fc_.as<float2>(), h, st);
       if (!r_zero) hk->adjoint_compact(r_.as<float2>(), z0, st, true);
-      launch_gram_start(W_, H_, static_cast<const float2*>(field(F_UB, p0)), k, U, st);
     }
     // reads {alpha0, alpha1} of row 0 whatever the row length
     launch_mri_dual(is_tgv, W_, H_, ptrs(p0), ptrs(p0 ^ 1), sigma, reinterpret_cast<const float*>(table), header, st);
@@ -892,10 +889,10 @@ class OptImpl {
       primal(g.src, par);
       primal(g.dst, par ^ 1);
       if (row_op) {
-        g.U = U + 2 * N * par;
-        g.Unext = U + 2 * N * (par ^ 1);
-        g.b = b;
-        g.b_lo = b_lo;
+        g.D = D + 2 * N * par;
+        g.Dnext = D + 2 * N * (par ^ 1);
+        g.w = w;
+        g.h = h;
         g.z0 = r_zero ? nullptr : z0;
       }
       g.part = part;
@@ -908,7 +905,7 @@ class OptImpl {
       g.lambda = lambda;
       g.k = k;
       if (row_op) {
-        launch_gram_rows(rows, g.U, part, s);
+        launch_gram_rows(rows, g.D, part, s);
         if (prof_) prof_->mark("mri_gram_rows", s);
       } else {
         hk->round(static_cast<const float2*>(field(F_UB, p0 ^ par)), r_.as<float2>(), fc_.as<float2>(), sigma, lambda,
@@ -922,14 +919,36 @@ class OptImpl {
         for (int f : {(int)F_U, (int)F_VX, (int)F_VY})
           if (f == F_U || is_tgv)
             PDT_CUDA_CHECK(cudaMemcpyAsync(raw_field(f, 0), raw_field(f, 1), plane, cudaMemcpyDeviceToDevice, s));
-      if (row_op) hk->dual_from_image(U + 2 * N * ((n - 1) & 1), r_.as<float2>(), fc_.as<float2>(), c, d, s);
+      if (row_op) {
+        launch_gram_total(W_, H_, D + 2 * N * ((n - 1) & 1), w, c, part, s);
+        hk->dual_from_image(part, r_.as<float2>(), fc_.as<float2>(), c, d, s);
+      }
       if (prof_) prof_->mark("mri_finish", s);
     };
     pl.key = graph_key({(uintptr_t)img_.p, (uintptr_t)gram_.p, (uintptr_t)khr_.p, (uintptr_t)r_.p, (uintptr_t)fc_.p,
                         (uintptr_t)alpha_.p, (uintptr_t)alpha_.bytes, (uintptr_t)op_.get(), (uintptr_t)op_->generation(),
                         (uintptr_t)W_, (uintptr_t)H_, (uintptr_t)groups, (uintptr_t)p0, (uintptr_t)is_tgv,
-                        (uintptr_t)r_zero, (uintptr_t)row_op, (uintptr_t)b_lo, fbits(lambda), fbits(tau), fbits(sigma),
+                        (uintptr_t)r_zero, (uintptr_t)row_op, fbits(lambda), fbits(tau), fbits(sigma),
                         (uintptr_t)version_, (uintptr_t)1});
+  }
+
+  // The row operator's planes: two copies of {D, compensation}, w, h, z0, partial sums, then kGramDots values; and the
+  // operator's scratch. False where the device has no room for them: round() needs less.
+  bool reserve_row_op(const GramRows& g, SolverHooks* hk) {
+    const size_t bytes = (7 + (size_t)g.groups) * plane_bytes() + kGramDots * sizeof(float2);
+    try {
+      if (gram_.bytes != bytes) {
+        ++version_;
+        gram_.ensure(bytes);
+      }
+      hk->reserve_residual();
+    } catch (const Error& e) {
+      if (e.code != PDT_ERR_ALLOC) throw;
+      cudaGetLastError();
+      gram_.release();
+      return false;
+    }
+    return true;
   }
 
   void ensure_fc(SolverHooks* hk, cudaStream_t st) {
@@ -982,8 +1001,16 @@ class OptImpl {
 
   static constexpr int kGraphIters = 20;
   static constexpr size_t kAlphaHeader = 64;
-  static constexpr unsigned kGramMinIters = 8;
-  static constexpr int kPairMinIters = 256;  // see plan_image() and pdt_cart_pair.cuh
+  // The row operator's set-up and the k-space dual at its end take 0.06 ms (2 coils, 64 x 64) to 0.47 ms (15 coils,
+  // 640 x 368), against what an iteration saves: paid back after 8 iterations or fewer (2 coils 64 x 64, 8 iterations 200
+  // us with either; 8 coils 231 x 175 330 / 614 us), 9 (20 coils 256 x 256, 363 / 329), 13 (15 coils, 320 x 368 rows,
+  // 12 iterations 599 / 570) and 16 (15 coils 640 x 368, 12 iterations 1029 / 890).
+  static constexpr int kGramMinIters = 8, kGramMinItersLarge = 13;
+  static constexpr size_t kGramLarge = (size_t)1 << 20;  // coil pixels
+  // Bound on c. Error against FP64 of the row operator / of the k-space dual, 1001 iterations of TGV, 4 coils 48 x 48
+  // (NumPy models in FP32): c = 4: 0.97e-7 / 1.60e-7, with maps scaled by 2.5 0.96e-7 / 0.98e-7; c = 8: 1.09e-7 / 1.13e-7,
+  // scaled 1.6e-7 / 0.9e-7; c = 125 (Lambda 0): 4.6e-7 / 1.4e-7.
+  static constexpr double kGramMaxC = 4;
 
   pdt_opt_kind kind_;
   bool cplx_;

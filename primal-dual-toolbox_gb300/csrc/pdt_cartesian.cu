@@ -431,32 +431,42 @@ class CartesianOp : public OpImpl, public SolverHooks {
       launch_rows_adj(t, khr, groups_run(), st);
     if (mk) mk->mark("cart_rows_adj", st);
   }
-  bool adjoint_pair(const float2* fc, float2* img, float2* lo, cudaStream_t st) override {
+  void reserve_residual() override {
     prepare();
-    int nq = std::min(4, dev_.C);
-    while (nq > 1 && pair_rows_smem(dev_.W, nq) > 100 * 1024) --nq;
-    const size_t cs = pair_cols_smem(dev_.Hf), rs = pair_rows_smem(dev_.W, nq), smem = std::max(cs, rs);
-    if (dev_.ns == 0 || smem > (size_t)g_max_smem) return false;
-    if (!pair_built_) {
-      std::vector<float4> h, w;
-      pair_twiddles(dev_.Hf, h);
-      pair_twiddles(dev_.W, w);
-      h.insert(h.end(), w.begin(), w.end());
-      pair_tab_.ensure(h.size() * sizeof(float4));
-      PDT_CUDA_CHECK(cudaMemcpy(pair_tab_.p, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
-      pair_t_.ensure((size_t)dev_.C * dev_.ns * dev_.Hi * sizeof(float4));
-      PDT_CUDA_CHECK(cudaFuncSetAttribute(pair_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
-      PDT_CUDA_CHECK(cudaFuncSetAttribute(pair_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
-      pair_built_ = true;
-    }
+    if (pair_built_) return;
+    std::vector<float4> h, w;
+    pair_twiddles(dev_.Hf, h);
+    pair_twiddles(dev_.W, w);
+    h.insert(h.end(), w.begin(), w.end());
+    pair_tab_.ensure(h.size() * sizeof(float4));
+    pair_t_.ensure((size_t)dev_.C * dev_.ns * dev_.Hi * sizeof(float4));
+    pair_p_.ensure((size_t)pair_groups(dev_.C, dev_.Hi, g_num_sms) * dev_.Hi * dev_.W * sizeof(float4));
+    PDT_CUDA_CHECK(cudaMemcpy(pair_tab_.p, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    PDT_CUDA_CHECK(cudaFuncSetAttribute(pair_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
+    PDT_CUDA_CHECK(cudaFuncSetAttribute(pair_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, g_max_smem));
+    // Not the largest share of shared memory, which pair_cols' occupancy would ask for: with several solves in flight the
+    // SMs kept that split, and its small L1, for the iterations that follow (three benchmark solves at a time 16.5 us an
+    // iteration instead of 15.5).
+    for (const void* fn : {(const void*)pair_cols, (const void*)pair_rows})
+      PDT_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 58));
+    pair_built_ = true;
+  }
+  void adjoint_residual(const float2* u, const float2* fc, float2* out, cudaStream_t st) override {
+    reserve_residual();
     const float4* tw = pair_tab_.as<float4>();
-    const float2 scale = pair_of(1.0 / std::sqrt((double)dev_.W * dev_.Hf));
-    pair_cols<<<dim3(dev_.ns, dev_.C), kPairThreads, cs, st>>>(dev_, tw, fc, pair_t_.as<float4>());
+    pair_cols<<<dim3(dev_.ns, dev_.C), kPairThreads, pair_cols_smem(dev_.Hf), st>>>(dev_, pair_planH_, tw, fc,
+                                                                                     pair_t_.as<float4>());
     PDT_LAUNCH_CHECK();
-    pair_rows<<<dev_.Hi, kPairThreads, rs, st>>>(dev_, tw + dev_.Hf, pair_t_.as<float4>(), nq, scale, img, lo);
+    const int G = pair_groups(dev_.C, dev_.Hi, g_num_sms), nq = pair_coils(dev_.C, G);
+    const size_t N = (size_t)dev_.Hi * dev_.W;
+    pair_rows<<<dim3(dev_.Hi, G), 64 * std::max(nq, 2), pair_rows_smem(dev_.W, nq), st>>>(
+        dev_, pair_planW_, tw + dev_.Hf, pair_t_.as<float4>(), u, nq, pair_of(std::sqrt((double)dev_.Hf / dev_.W)),
+        pair_p_.as<float4>());
     PDT_LAUNCH_CHECK();
-    count_launch(2);
-    return true;
+    pair_sum<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(N, pair_p_.as<float4>(), G,
+                                                          pair_of(1.0 / std::sqrt((double)dev_.W * dev_.Hf)), out);
+    PDT_LAUNCH_CHECK();
+    count_launch(3);
   }
   void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool exact_rows) override {
     prepare();
@@ -882,7 +892,8 @@ class CartesianOp : public OpImpl, public SolverHooks {
   }
 
   // The solvers' row operator (pdt_gram.h) where every sampled column of the mask is constant along the
-  // readout. A pinned tuning pins the three-pass round as well.
+  // readout and the pair transforms of adjoint_residual() fit shared memory. A pinned tuning pins the three-pass
+  // round as well.
   void prepare_gram(const float* mask, const std::vector<int>& col_x) {
     gram_ = GramRows();
     const char* pin = std::getenv("PDT_CARTESIAN_TUNE");
@@ -891,7 +902,9 @@ class CartesianOp : public OpImpl, public SolverHooks {
       for (int x : col_x)
         if (!(mask[(size_t)y * dev_.W + x] == mask[x])) return;
     const GramLength len = gram_length(dev_.W);
-    if (!len.n) return;
+    if (!len.n || !pair_plan(dev_.Hf, &pair_planH_) || !pair_plan(dev_.W, &pair_planW_) ||
+        std::max(pair_cols_smem(dev_.Hf), pair_rows_smem(dev_.W, kPairCoils)) > (size_t)g_max_smem)
+      return;
     std::vector<float> m2(dev_.W, 0.f), spec;
     for (int x : col_x) m2[(x + dev_.W - dev_.oxW) % dev_.W] = mask[x] * mask[x];  // DFT index of column x
     std::vector<float2> tw;
@@ -1112,7 +1125,8 @@ class CartesianOp : public OpImpl, public SolverHooks {
   bool prepared_ = false;
   RowFft row_fft_;
   bool row_fft_ok_ = false, pinned_ = false;
-  DevBuf pair_tab_, pair_t_;  // adjoint_pair(): twiddles of Hf and W, columns of [c][s][yi]
+  DevBuf pair_tab_, pair_t_, pair_p_;  // adjoint_residual(): twiddles of Hf and W, columns, coil groups' images
+  FftPlan pair_planH_{}, pair_planW_{};
   bool pair_built_ = false;
   Tune tune_;
   CartDev dev_{};

@@ -21,12 +21,12 @@ struct RowsArgs {
   size_t coil_stride;
   const float2* tw;
   const float* spec;
-  const float2* U;
+  const float2* D;
   float2* part;
 };
 
 // Block (g, y): row y, coil group g, in passes of up to CB coils. Per pass, with a block barrier between,
-//   1  per coil and t < Q: s_c . U at x = t + Q j (j < P), P-point DFT            -> Y[c][k1][t]
+//   1  per coil and t < Q: s_c . D at x = t + Q j (j < P), P-point DFT            -> Y[c][k1][t]
 //   2  per coil and k1 < P: twiddle, Q-point DFT, times the spectrum of G, inverse -> Y[c][k1][t]
 //   3  per coil and t: inverse P-point DFT, times conj(s_c)                         -> Y[c][j][t]
 //   4  sum over the pass's coils in coil order
@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
   const int cb = (int)((long long)blockIdx.x * a.C / gridDim.x), ce = (int)((long long)(blockIdx.x + 1) * a.C / gridDim.x);
   const bool two = ce - cb > a.CB;
   float2* tws = gsm;                                          // [Q][P]
-  float2* Us = tws + n;                                       // [n], zero past W
-  float2* Y = Us + n;                                         // [CB][P][LD]
+  float2* Ds = tws + n;                                       // [n], zero past W
+  float2* Y = Ds + n;                                         // [CB][P][LD]
   float2* S = Y + a.CB * (P * LD);                            // one or two of [CB][n], zero past W
   float* spec = reinterpret_cast<float*>(S + (a.sens ? (two ? 2 : 1) * a.CB * n : 0));  // [n]
   auto stage = [&](int c0, float2* dst) {
@@ -62,14 +62,14 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
     spec[i] = a.spec[i];
   }
   if (W < n) {
-    for (int x = W + tid; x < n; x += kGramThreads) Us[x] = c2(0.f, 0.f);
+    for (int x = W + tid; x < n; x += kGramThreads) Ds[x] = c2(0.f, 0.f);
     if (a.sens)
       for (int c = 0; c < (two ? 2 : 1) * a.CB; ++c)
         for (int x = W + tid; x < n; x += kGramThreads) S[c * n + x] = c2(0.f, 0.f);
   }
-  pdl_wait();  // everything above is constant; U comes from the previous kernel
+  pdl_wait();  // everything above is constant; D comes from the previous kernel
   pdl_trigger();
-  for (int x = tid; x < W; x += kGramThreads) Us[x] = a.U[(size_t)y * W + x];
+  for (int x = tid; x < W; x += kGramThreads) Ds[x] = a.D[(size_t)y * W + x];
   float2 z[KX];
 #pragma unroll
   for (int k = 0; k < KX; ++k) z[k] = c2(0.f, 0.f);
@@ -87,10 +87,10 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
       if (a.sens) {
         const float2* s = sc + c * n + t;
 #pragma unroll
-        for (int j = 0; j < P; ++j) v[j] = cmul(Us[t + Q * j], s[Q * j]);
+        for (int j = 0; j < P; ++j) v[j] = cmul(Ds[t + Q * j], s[Q * j]);
       } else {
 #pragma unroll
-        for (int j = 0; j < P; ++j) v[j] = Us[t + Q * j];
+        for (int j = 0; j < P; ++j) v[j] = Ds[t + Q * j];
       }
       float2* yc = Y + c * (P * LD) + t;
       cfft_out<P, -1>(v, [&](auto K, float2 o) { yc[decltype(K)::value * LD] = o; });
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
 // ------------------------------------------------------------------------------------------------
 // Image side of an iteration for a 32 x 8 tile: the primal update on the tile and one column and row beyond
 // it (the next dual update reads ubar and vbar at x + 1 and y + 1), from the p, q of the tile and its
-// halo; then the dual update and U of the next iteration. Everything but K^H K U is complete before the
+// halo; then the dual update and D of the next iteration. Everything but K^H K D is complete before the
 // row kernel starts, and nothing the row kernel reads is written here, so the divergences, the v update and
 // the next q run before the programmatic wait (L2 loads: this SM may hold older lines). Bound by the latency
 // of its load phases: four blocks an SM (48 registers, some spilled) make one wave of the 480 blocks of a
@@ -189,24 +189,16 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   const bool in = tid < (GX + 1) * (GY + 1) && x < W && y < H;
   const bool own = in && lx < GX && ly < GY;
   const size_t idx = in ? (size_t)y * W + x : 0;
-  float2 ou = c2(0.f, 0.f), kf = ou, ke = ou, ovx = ou, ovy = ou, Uo = ou, Ue = ou;
+  float2 ou = c2(0.f, 0.f), kf = ou, ovx = ou, ovy = ou;
   if (in) {
     ou = ld(s.src.u, idx);
     if constexpr (ROWS) {
-      // c K^H f as the rounded product and the rest: both it and K^H K U are far larger than their difference
-      const float2 b = __ldcg(s.b + idx);
-      kf = c2(__fmul_rn(row.z, b.x), __fmul_rn(row.z, b.y));
-      ke = c2(__fmaf_rn(row.z, b.x, -kf.x), __fmaf_rn(row.z, b.y, -kf.y));
-      if (s.b_lo) ke = ke + row.z * __ldcg(s.b_lo + idx);
-      if (s.z0) ke = ke - row.w * __ldcg(s.z0 + idx);
+      kf = row.z * __ldcg(s.h + idx);
+      if (s.z0) kf = kf + row.w * __ldcg(s.z0 + idx);
     }
     if constexpr (TGV) {
       ovx = ld(s.src.vx, idx);
       ovy = ld(s.src.vy, idx);
-    }
-    if (ROWS && own) {
-      Uo = __ldcg(s.U + idx);
-      Ue = __ldcg(s.U + (size_t)W * H + idx);
     }
   }
   __syncthreads();
@@ -253,13 +245,19 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
       static_cast<float2*>(s.dst.qxy)[idx] = qc * sq;
     }
   }
-  pdl_wait();  // K^H K U comes from the row kernel
+  pdl_wait();  // K^H K D comes from the row kernel
   pdl_trigger();
   if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) s.header[4 + (s.par ^ 1)] = it + 1;
+  float2 Do = c2(0.f, 0.f), De = Do, w = Do;
+  if (ROWS && own) {  // in flight together with the sums (earlier they would only hold registers)
+    Do = __ldcg(s.D + idx);
+    De = __ldcg(s.D + (size_t)W * H + idx);
+    w = __ldcg(s.w + idx);
+  }
   if (in) {
     float2 kh = s.part[idx];
     for (int g = 1; g < s.groups; ++g) kh += s.part[idx + (size_t)g * W * H];
-    if constexpr (ROWS) kh = (kh - kf) - ke;
+    if constexpr (ROWS) kh = kh + kf;
     const float2 un = ou + s.tau * (dp - kh);
     s_ub[ly][lx] = 2.0f * un - ou;
     finite = finite && isfinite(un.x) && isfinite(un.y);
@@ -282,24 +280,66 @@ __global__ void __launch_bounds__(GT, 4) gram_image_kernel(GramImage s) {
   static_cast<float2*>(s.dst.px)[idx] = a * sp;
   static_cast<float2*>(s.dst.py)[idx] = b * sp;
   if constexpr (!ROWS) return;
-  // U + its compensation
-  auto step = [&](float u, float e, float ub, float& nu, float& ne) {
-    const float inc = __fadd_rn(e, s.k * ((ub - s.lambda * u) - s.lambda * e));
-    nu = __fadd_rn(u, inc);
-    ne = __fsub_rn(inc, __fsub_rn(nu, u));
+  // D + its compensation
+  auto step = [&](float d, float e, float ub, float& nd, float& ne) {
+    const float inc = __fadd_rn(e, s.k * ((ub - s.lambda * d) - s.lambda * e));
+    nd = __fadd_rn(d, inc);
+    ne = __fsub_rn(inc, __fsub_rn(nd, d));
   };
-  float2 nu, ne;
-  step(Uo.x, Ue.x, c.x, nu.x, ne.x);
-  step(Uo.y, Ue.y, c.y, nu.y, ne.y);
-  s.Unext[idx] = nu;
-  s.Unext[(size_t)W * H + idx] = ne;
+  float2 nd, ne;
+  step(Do.x, De.x, c.x - w.x, nd.x, ne.x);
+  step(Do.y, De.y, c.y - w.y, nd.y, ne.y);
+  s.Dnext[idx] = nd;
+  s.Dnext[(size_t)W * H + idx] = ne;
 }
 
-__global__ void gram_start_kernel(size_t n, const float2* __restrict__ ubar, float k, float2* __restrict__ U) {
-  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+constexpr int kStartThreads = 256;
+
+// dots[block] = {|w|^2, Re <w, K^H K w>} over every kGramDots-th run of pixels.
+__global__ void __launch_bounds__(kStartThreads) gram_dots_kernel(size_t n, const float2* __restrict__ w,
+                                                                  const float2* __restrict__ part, int groups,
+                                                                  float2* __restrict__ dots) {
+  __shared__ float2 sh[kStartThreads];
+  float2 s = c2(0.f, 0.f);
+  for (size_t i = blockIdx.x * (size_t)kStartThreads + threadIdx.x; i < n; i += (size_t)kGramDots * kStartThreads) {
+    float2 g = part[i];
+    for (int q = 1; q < groups; ++q) g += part[i + q * n];
+    const float2 v = w[i];
+    s += c2(abs2(v), v.x * g.x + v.y * g.y);
+  }
+  sh[threadIdx.x] = s;
+  for (int o = kStartThreads / 2; o > 0; o >>= 1) {
+    __syncthreads();
+    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  }
+  if (threadIdx.x == 0) dots[blockIdx.x] = sh[0];
+}
+
+__global__ void __launch_bounds__(kStartThreads) gram_start_kernel(size_t n, const float2* __restrict__ dots,
+                                                                   const float2* __restrict__ ubar, float k,
+                                                                   float2* __restrict__ w, float2* __restrict__ D) {
+  __shared__ float2 sh[kGramDots];
+  if (threadIdx.x < kGramDots) sh[threadIdx.x] = dots[threadIdx.x];
+  for (int o = kGramDots / 2; o > 0; o >>= 1) {
+    __syncthreads();
+    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  }
+  __syncthreads();
+  float a = sh[0].x / sh[0].y;
+  if (!isfinite(a)) a = 0.f;
+  const size_t i = blockIdx.x * (size_t)kStartThreads + threadIdx.x;
   if (i >= n) return;
-  U[i] = k * ubar[i];
-  U[n + i] = c2(0.f, 0.f);
+  const float2 v = a * w[i];
+  w[i] = v;
+  D[i] = k * (ubar[i] - v);
+  D[n + i] = c2(0.f, 0.f);
+}
+
+__global__ void __launch_bounds__(kStartThreads) gram_total_kernel(size_t n, const float2* __restrict__ D,
+                                                                   const float2* __restrict__ w, float c,
+                                                                   float2* __restrict__ out) {
+  const size_t i = blockIdx.x * (size_t)kStartThreads + threadIdx.x;
+  if (i < n) out[i] = c2(fmaf(c, w[i].x, D[i].x), fmaf(c, w[i].y, D[i].y));
 }
 
 typedef void (*GramFn)(RowsArgs);
@@ -392,14 +432,14 @@ void gram_tables(int W, const GramLength& len, const std::vector<float>& m2, std
   }
 }
 
-void launch_gram_rows(const GramRows& g, const float2* U, float2* part, cudaStream_t st) {
+void launch_gram_rows(const GramRows& g, const float2* D, float2* part, cudaStream_t st) {
   for (const auto& k : kGramKernels) {
     if (k.len.n != g.len.n || k.len.P != g.len.P) continue;
     const int per = (g.C + g.groups - 1) / g.groups;  // coils of the largest group, in equal passes
     const int passes = (per + gram_pass(g.len) - 1) / gram_pass(g.len);
     const int CB = (per + passes - 1) / passes;
     const size_t smem = gram_smem(g.len, CB, g.sens ? (passes > 1 ? 2 : 1) : 0);
-    const RowsArgs a{g.W, g.H, g.C, CB, g.sens, g.coil_stride, g.tw, g.spec, U, part};
+    const RowsArgs a{g.W, g.H, g.C, CB, g.sens, g.coil_stride, g.tw, g.spec, D, part};
     PDT_CUDA_CHECK(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     LaunchEx lx(dim3(g.groups, g.H), dim3(kGramThreads), smem, st);
     PDT_CUDA_CHECK(cudaLaunchKernelEx(&lx.cfg, k.fn, a));
@@ -417,9 +457,19 @@ void launch_gram_image(bool tgv, bool rows, const GramImage& s, cudaStream_t st)
   count_launch();
 }
 
-void launch_gram_start(int W, int H, const float2* ubar, float k, float2* U, cudaStream_t st) {
+void launch_gram_start(int W, int H, const float2* part, int groups, const float2* ubar, float k, float2* w, float2* D,
+                       float2* dots, cudaStream_t st) {
   const size_t n = (size_t)W * H;
-  gram_start_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, ubar, k, U);
+  gram_dots_kernel<<<kGramDots, kStartThreads, 0, st>>>(n, w, part, groups, dots);
+  PDT_LAUNCH_CHECK();
+  gram_start_kernel<<<(unsigned)((n + kStartThreads - 1) / kStartThreads), kStartThreads, 0, st>>>(n, dots, ubar, k, w, D);
+  PDT_LAUNCH_CHECK();
+  count_launch(2);
+}
+
+void launch_gram_total(int W, int H, const float2* D, const float2* w, float c, float2* out, cudaStream_t st) {
+  const size_t n = (size_t)W * H;
+  gram_total_kernel<<<(unsigned)((n + kStartThreads - 1) / kStartThreads), kStartThreads, 0, st>>>(n, D, w, c, out);
   PDT_LAUNCH_CHECK();
   count_launch();
 }

@@ -59,9 +59,10 @@ struct SolverHooks {
   // `exact_rows`: with row transforms whose error is that of FP32 rounding also where another kernel (TF32
   // triples, about 1e-6 relative) is faster.
   virtual void adjoint_compact(const float2* fc, float2* img, cudaStream_t st, bool exact_rows = false) = 0;
-  // The same as a sum of two FP32 images, accurate to FP64 rounding of the data; false (and nothing done) where the
-  // operator has no such adjoint.
-  virtual bool adjoint_pair(const float2* /*fc*/, float2* /*img*/, float2* /*lo*/, cudaStream_t /*st*/) { return false; }
+  // With line_gram(): out <- K^H (K u - f), its error that of rounding the result to FP32 (pdt_cart_pair.cuh); and its
+  // scratch, which a solve asks for before it chooses the row operator (throws PDT_ERR_ALLOC).
+  virtual void adjoint_residual(const float2* /*u*/, const float2* /*fc*/, float2* /*out*/, cudaStream_t /*st*/) {}
+  virtual void reserve_residual() {}
 };
 
 class OpImpl {
