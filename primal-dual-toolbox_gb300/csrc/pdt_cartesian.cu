@@ -298,7 +298,10 @@ class CartesianOp : public OpImpl, public SolverHooks {
   void dual_from_image(const float2* U, float2* r, const float2* fc, float c, float d, cudaStream_t st) override {
     prepare();
     float2* t = scratch_.as<float2>();
-    launch_rows_fwd(U, t, nullptr, st);
+    if (row_fft_ok_ && !pinned_)
+      launch_row_fft_fwd(row_fft_, U, t, nullptr, nullptr, 0, st);
+    else
+      launch_rows_fwd(U, t, nullptr, st, true);
     launch_cols(COL_DUAL, t, nullptr, r, fc, nullptr, nullptr, c, d, st);
   }
   void check_device_errors() override {
@@ -632,8 +635,9 @@ class CartesianOp : public OpImpl, public SolverHooks {
   bool ra() const { return tune_.ra != 0; }
   bool tcf() const { return tune_.tcf && !(concurrent_ && frow_.ok()); }
 
-  void launch_rows_fwd(const float2* ubar, float2* t1, int* tick, cudaStream_t st) {
-    if (tcf()) {
+  // `exact`: in FP32 (the tensor-core rows carry 22 bits).
+  void launch_rows_fwd(const float2* ubar, float2* t1, int* tick, cudaStream_t st, bool exact = false) {
+    if (tcf() && !exact) {
       launch_tc_rows_fwd(ubar, t1, tick, st);
       return;
     }

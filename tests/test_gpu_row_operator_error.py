@@ -61,3 +61,31 @@ def test_error_is_that_of_the_k_space_dual(pdt, oracle, case, model):
     sampled = (d["mask"] != 0).any(axis=0)
     r = state["r"].reshape(f.shape)
     assert np.linalg.norm((o.getField("r") - r)[:, :, sampled]) <= 1e-5 * np.linalg.norm(f)
+
+
+def test_k_space_dual_at_the_end_has_fp32_rows(pdt, oracle):
+    """Where the tuner keeps the tensor-core forward rows (TF32 triples, about 1e-6 off), r = K U - c f must not take
+    them. The NumPy model's r is 1.23e-7 of |f| off after these 40 iterations; twice that."""
+    from primaldualtoolbox import synthetic
+
+    C, H, W = 8, 320, 250
+    d = synthetic.cartesian_case(C=C, H=H, W=W, roos=False, seed=0, accel=4)
+    op = pdt.mri.MriCartesianOperator()
+    op.setCoilSens(d["sens"])
+    op.setMask(d["mask"])
+    if "rows_fwd=tensor_dft" not in op.tuning():
+        pytest.skip("the tuner chose FP32 rows")
+    o = pdt.mri.TgvMriOptimizer_2c3c()
+    prm = o.getParameters()
+    a1 = float(np.float32(d["alpha1"]))
+    prm.max_iter, prm.reduction, prm.alpha1, prm.alpha0 = 39, 1.0, a1, 2 * a1
+    o.setOperator(op)
+    o.setNoisyData(d["rawdata"])
+    u0 = op.adjoint(d["rawdata"])
+    o.setInput0(u0)
+    o.solve()
+    _, state = oracle.op_solve("cartesian", d["sens"], d["mask"], d["rawdata"], "tgv_mri", alpha0=2 * a1, alpha1=a1,
+                               reduction=1.0, max_iter=39, u0=u0, prec=64, return_state=True)
+    sampled = (d["mask"] != 0).any(axis=0)
+    diff = (o.getField("r") - state["r"].reshape(C, H, W))[:, :, sampled]
+    assert np.linalg.norm(diff) <= 2.5e-7 * np.linalg.norm(d["rawdata"])
