@@ -33,7 +33,7 @@ struct DenoiseArgs {
   int W, H, halo, steps, store_bar;
   ImgPtrs in, out;
   const void* f;
-  float tau, sigma, lambda, alpha0, alpha1;
+  float tau, sigma, lambda, alpha0, alpha1, inside0, inside1;  // see proj()
 };
 
 template <class P, bool TGV, int RX, int RY, int SR, int MINB>
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(RX* RY / SR, MINB) denoise_kernel(DenoiseArgs 
   }
   const float inv = 1.0f / (1.0f + a.tau * a.lambda);
   const float a1 = TGV ? a.alpha1 : 1.0f;
-  const float in0 = a.alpha0 * a.alpha0 * (1.0f - 0x1p-20f), in1 = a1 * a1 * (1.0f - 0x1p-20f);
+  const float in0 = a.inside0, in1 = a.inside1;
   // div- along x of a plane at row j (its value c there) and along y from the value above
   auto dx = [&](P c, const P* s, int j) {
     const P l = s[(ly + j) * RX + lx - 1];
@@ -268,7 +268,11 @@ int denoise_steps(bool complex_, bool tgv, int W, int H, int iters, int* region)
 void launch_denoise(bool complex_, bool tgv, int W, int H, const ImgPtrs& in, const ImgPtrs& out, const void* f, float tau,
                     float sigma, float lambda, float alpha0, float alpha1, int region, int halo, int steps,
                     bool store_bar, cudaStream_t st) {
-  const DenoiseArgs a{W, H, halo, steps, store_bar ? 1 : 0, in, out, f, tau, sigma, lambda, alpha0, alpha1};
+  // the shortcut of proj() only where alpha^2 neither overflows (with n2 = inf the result is 0) nor loses bits to underflow
+  auto inside = [](float al) { return al >= 0x1p-60f && al <= 0x1p60f ? al * al * (1.0f - 0x1p-20f) : -1.0f; };
+  const DenoiseArgs a{W,     H,      halo,   steps,  store_bar ? 1 : 0, in,
+                      out,   f,      tau,    sigma,  lambda,            alpha0,
+                      alpha1, inside(alpha0), inside(tgv ? alpha1 : 1.0f)};
   if (complex_)
     tgv ? launch_any<float2, true>(region, a, st) : launch_any<float2, false>(region, a, st);
   else

@@ -46,3 +46,18 @@ def test_regions_match_oracle(pdt, oracle, H, W, cplx, tgv):
             o.setInput0UV(f)
             o.solve()
             assert rel_l2(q, 2 * np.asarray(ref) - o.getResult()) <= TOL
+
+
+def test_projection_of_overflowing_duals(pdt, oracle):
+    """|p|^2 beyond FP32's range and alpha^2 too: 1 / max(1, inf / alpha) = 0. The FP32 oracle evaluates the same
+    expression; four iterations of a few roundings of 2^-24 each stay within 1e-6."""
+    rng = np.random.default_rng(5)
+    f = (1e21 * rng.standard_normal((40, 48))).astype(np.float32)
+    opt = pdt.denoising.TgvOptimizer_2f()
+    prm = opt.getParameters()
+    prm.max_iter, prm.Lambda, prm.alpha0, prm.alpha1 = 3, 10.0, 1e20, 1e20
+    opt.setNoisyData(f)
+    opt.solve()
+    ref = oracle.tgv_solve(f, lam=10.0, alpha0=1e20, alpha1=1e20, max_iter=3, prec=32)
+    assert np.isfinite(ref).all()
+    assert rel_l2(opt.getResult(), ref) <= 1e-6
