@@ -891,6 +891,10 @@ class CartesianOp : public OpImpl, public SolverHooks {
     tune_.rf = tune_.ra = row_fft_ok_;  // where nothing is tuned: against the generic rows
     autotune();
     dev_ = d;
+    if (const char* env = std::getenv("PDT_REGISTER_ROWS"); env && std::atoi(env) && row_fft_ok_ && !pinned_) {
+      tune_.rf = tune_.ra = 1;  // whatever the tuner measured
+      tune_.tcf = tune_.tca = 0;
+    }
     prepare_gram(mask, col_x);
     prepared_ = true;
   }
