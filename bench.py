@@ -186,9 +186,20 @@ def _phase_bytes_case(C, Hf, W, ns, G, roos):
 
 def _line_gram_bytes(N, C, sums):
     """Algorithmic bytes per launch of a line-sampled solve's two kernels (N image pixels, C coils, `sums`
-    coil-group sums of K^H K U): the row operator reads U and the maps and writes the sums; the image kernel reads
-    u, v(2), p(2), q(3), K^H f, U with its compensation and the sums and writes u, v, p, q and U again."""
-    return {"mri_gram_rows": 8 * N * (1 + C + sums), "mri_image_tgv": 8 * N * (8 + 1 + 2 + sums + 8 + 2)}
+    coil-group sums of K^H K D): the row operator reads D and the maps and writes the sums; the image kernel reads
+    u, v(2), p(2), q(3), the reference image, K^H of its residual, D with its compensation and the sums and writes u, v,
+    p, q and D again."""
+    return {"mri_gram_rows": 8 * N * (1 + C + sums), "mri_image_tgv": 8 * N * (8 + 2 + 2 + sums + 8 + 2)}
+
+
+# Iterations a launch of the denoising kernels takes on images of 131072 pixels and more (denoise_steps).
+DENOISE_STEPS = 3
+
+
+def _denoise_planes(tgv):
+    """Image planes that one iteration moves, DENOISE_STEPS of them a launch: a TV launch reads u, u-bar, p(2), f and
+    writes u, u-bar, p(2); a TGV launch reads u, v(2), p(2), q(3), f and writes u, v, p, q."""
+    return (17 if tgv else 9) / DENOISE_STEPS
 
 
 def _coil_sums(tuning):
@@ -832,16 +843,16 @@ def run_radial(pdt, torch, slices, iters, converge=True):
 
 def run_denoising(pdt, torch, reps=3):
     """Config 1 (TvOptimizer, 512 x 512 float32, lambda 10, 500 -> 501 iterations) and the same image
-    through TgvOptimizer (alpha1 0.1, alpha0 0.2), data resident. Algorithmic bytes per iteration of the
-    fused kernels: TV reads u-bar, p (2), u, f and writes p (2), u, u-bar = 9 planes (+ 2 halo re-reads
-    not counted); TGV 12 reads + 11 writes of the 11-plane state (f included) = 23 planes."""
+    through TgvOptimizer (alpha1 0.1, alpha0 0.2), data resident. Algorithmic bytes per iteration as in
+    _denoise_planes (halo re-reads not counted)."""
     from primaldualtoolbox import synthetic
 
     f = torch.from_numpy(synthetic.tv_phantom(512, 512, seed=0)[0]).cuda()  # the noisy image
     stream = torch.cuda.current_stream()
     hbm, src = _peaks()
     out = {}
-    for name, cls, planes in (("tv_rof", pdt.denoising.TvOptimizer_2f, 9), ("tgv", pdt.denoising.TgvOptimizer_2f, 23)):
+    for name, cls, planes in (("tv_rof", pdt.denoising.TvOptimizer_2f, _denoise_planes(False)),
+                              ("tgv", pdt.denoising.TgvOptimizer_2f, _denoise_planes(True))):
         opt = cls()
         prm = opt.getParameters()
         prm.max_iter, prm.Lambda = 500, 10.0
@@ -857,7 +868,7 @@ def run_denoising(pdt, torch, reps=3):
         e1.record(stream)
         torch.cuda.synchronize()
         dt = e0.elapsed_time(e1) / 1e3 / reps
-        nbytes = 4 * 512 * 512 * planes
+        nbytes = int(4 * 512 * 512 * planes)
         out[name] = {"value": round(501 / dt, 1), "unit": "iters/s", "ms_per_solve": round(dt * 1e3, 3),
                      "roofline": {"bound": "hbm", "achieved": round(nbytes * 501 / dt / 1e9, 1), "peak": hbm,
                                   "peak_source": src, "unit": "GB/s",
@@ -872,16 +883,16 @@ def run_denoising_hbm(pdt, torch, reps=3, iters=21):
     """The fused primal-dual step kernels on HBM-resident images (the 512 x 512 benchmark image's state
     fits in L2): TV and TGV on an 8192 x 8192 float32 image (TGV state 2 x 11 planes = 5.6 GB) and TGV on a
     complex 8192 x 4096 image, each a seeded phantom tiled to size, `iters` iterations per solve. Bytes per
-    iteration as run_denoising (TV 9 planes, TGV 23 planes of the pixel type)."""
+    iteration as run_denoising."""
     from primaldualtoolbox import synthetic
 
     base = synthetic.tv_phantom(512, 512, seed=0)[0].astype(np.float32)
     stream = torch.cuda.current_stream()
     hbm, src = _peaks()
     out = {}
-    cases = (("tv_rof_8192x8192_f32", pdt.denoising.TvOptimizer_2f, 9, (8192, 8192), False),
-             ("tgv_8192x8192_f32", pdt.denoising.TgvOptimizer_2f, 23, (8192, 8192), False),
-             ("tgv_8192x4096_c64", pdt.denoising.TgvOptimizer_2c, 23, (8192, 4096), True))
+    cases = (("tv_rof_8192x8192_f32", pdt.denoising.TvOptimizer_2f, _denoise_planes(False), (8192, 8192), False),
+             ("tgv_8192x8192_f32", pdt.denoising.TgvOptimizer_2f, _denoise_planes(True), (8192, 8192), False),
+             ("tgv_8192x4096_c64", pdt.denoising.TgvOptimizer_2c, _denoise_planes(True), (8192, 4096), True))
     for name, cls, planes, (Hh, Ww), cplx in cases:
         img = np.tile(base, (Hh // 512, Ww // 512))
         if cplx:
@@ -902,15 +913,14 @@ def run_denoising_hbm(pdt, torch, reps=3, iters=21):
         e1.record(stream)
         torch.cuda.synchronize()
         dt = e0.elapsed_time(e1) / 1e3 / reps / iters
-        nbytes = (8 if cplx else 4) * Hh * Ww * planes
+        nbytes = int((8 if cplx else 4) * Hh * Ww * planes)
         out[name] = {"ms_per_iteration": round(dt * 1e3, 4),
                      "roofline": {"bound": "hbm", "achieved": round(nbytes / dt / 1e9, 1), "peak": hbm,
                                   "peak_source": src, "unit": "GB/s", "frac": round(nbytes / dt / 1e9 / hbm, 4),
                                   "algorithmic_bytes_per_iteration": nbytes}}
         del opt, f
-    out["note"] = ("TV runs four iterations per launch (temporal blocking in shared memory), so its bytes per "
-                   "iteration are the algorithmic ones of one iteration while the kernel passes over the state once "
-                   "per four")
+    out["note"] = (f"{DENOISE_STEPS} iterations a launch: the state passes memory once per launch, the bytes per "
+                   "iteration are that share of a launch's (the last launch's extra stores not counted)")
     return out
 
 

@@ -60,3 +60,13 @@ def test_khr_planes_from_the_tuning_report(bench):
     assert bench._batch_khr_planes(cluster) == (1, True)
     # an operator without lane-FFT rows (no in_batch report) keeps its solo figure
     assert bench._batch_khr_planes("rows_adj=stockham(coil_groups=3)") == (3, False)
+
+
+def test_denoising_bytes_are_those_of_a_launch_of_several_iterations(bench):
+    import re
+
+    src = open(os.path.join(ROOT, "primal-dual-toolbox_gb300", "csrc", "pdt_denoise.cu")).read()
+    steps = int(re.search(r"return std::min\((\d+), iters\);\n}\n", src).group(1))  # the rule's last line: large images
+    assert bench.DENOISE_STEPS == steps
+    # planes a launch stores and loads, once per `steps` iterations
+    assert bench._denoise_planes(False) * steps == 9 and bench._denoise_planes(True) * steps == 17
