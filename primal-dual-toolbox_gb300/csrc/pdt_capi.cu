@@ -762,7 +762,8 @@ class OptImpl {
     for (int k = 0; k < n && gc_last <= kGramMaxC; ++k) gc_last += (double)gk * (1.0 - (double)lambda * gc_last);
     // A line mask: an iteration is two launches (pdt_gram.h).
     const GramRows* gram = n >= kGramMinIters && gc_last <= kGramMaxC ? hk->line_gram() : nullptr;
-    if (gram && n < kGramMinItersLarge && (size_t)gram->C * gram->W * gram->H >= kGramLarge) gram = nullptr;
+    // (a profile of a few iterations shows the kernels of a solve of many)
+    if (gram && !profiling_ && n < kGramMinItersLarge && (size_t)gram->C * gram->W * gram->H >= kGramLarge) gram = nullptr;
     if (gram && !reserve_row_op(*gram, hk)) gram = nullptr;
     const int G = hk->groups();
     const long long gstride = hk->group_stride();
