@@ -255,6 +255,13 @@ void launch_any(int region, const DenoiseArgs& a, cudaStream_t st) {
 // Large images run on regions with more pixels a thread and more blocks an SM (512 x 512 TV c64: region 1 1.59,
 // region 0 1.73; 4096 x 4096 TGV f32: region 2 132, 1 134, 0 142); there the instructions bound it (square roots,
 // divisions, neighbours), not the 17 planes a launch.
+// The lines lie where a count of blocks passes a whole wave, which depends on the sides rather than the area. Both sides,
+// us an iteration of 121 back to back, TV f32 / TGV f32 / TV c64 / TGV c64:
+//   181^2  8: 0.77 1.19 0.88 1.56   6: 0.84 1.25 0.97 1.69      200^2  8: 0.97 1.66 1.19 2.76   6: 0.83 1.25 0.96 1.69
+//   362^2  6: 1.37 2.58 1.90 4.49   3: 1.44 2.34 1.88 3.81      400^2  6: 1.40 2.62 1.95 4.56   3: 1.77 2.39 2.32 3.95
+//   632^2  region 0, f32: 2.69 5.02   1 or 2: 2.62 4.84          720^2  region 0, f32: 3.14 5.98   1 or 2: 3.10 5.86
+// Four iterations are faster than the rule's number in some waves between (256^2 TGV f32 1.45 against 1.78, 448^2 TV f32
+// 1.59 against 1.83, 720^2 TGV f32 5.31 against 5.86): the rule does not count blocks.
 int denoise_steps(bool complex_, bool tgv, int W, int H, int iters, int* region) {
   const size_t n = (size_t)W * H;
   *region = 0;

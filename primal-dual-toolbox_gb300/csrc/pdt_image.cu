@@ -15,8 +15,8 @@ constexpr int NT = TX * TY;
 
 // ------------------------------------------------------------------------------------------------
 // TgvMriOptimizer / TgvOptimizerWithOp / TvOptimizerWithOp image side (dual first, K^H r given), as two
-// kernels so that the dual update runs concurrently with the operator chain (it needs only u-bar and
-// v-bar of the previous iteration):
+// kernels: the dual one runs a solve's first dual update (the others belong to the image kernel of pdt_gram.cu, or to
+// spare blocks of the operator's adjoint launch), the primal one every primal update of the latter route:
 //   dual    p <- proj_a1(p + sigma (grad+ ub - vb)),  q <- proj_a0(q + sigma eps(vb))   (in -> out)
 //   primal  u+ = u + tau (div- p - K^H r),            v+ = v + tau (div_h- q + p)       (p, q from out)
 // u and v are read only at their own pixel and update in place; u-bar and v-bar go to `out`.

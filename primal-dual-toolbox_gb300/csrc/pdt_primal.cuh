@@ -68,15 +68,10 @@ __device__ __forceinline__ void dual_alphas(const float* __restrict__ alpha_tab,
   }
 }
 
-// The dual values p, q of one pixel.
-struct DualVals {
-  float2 px, py, qxx, qyy, qxy;
-};
-
-// The updated dual values at pixel (x, y) from the u-bar, v-bar, p, q of `in`.
+// The dual update at pixel (x, y): u-bar, v-bar, p, q from `in`; p, q to `out`.
 template <bool TGV>
-__device__ __forceinline__ DualVals mri_dual_values(int W, int H, const ImgPtrs& in, float sigma, float alpha0,
-                                                    float alpha1, int x, int y) {
+__device__ __forceinline__ void mri_dual_pixel(int W, int H, const ImgPtrs& in, const ImgPtrs& out, float sigma,
+                                               float alpha0, float alpha1, int x, int y) {
   const size_t idx = (size_t)y * W + x;
   const bool xn = x < W - 1, yn = y < H - 1;
   const float2* ub = static_cast<const float2*>(in.ub);
@@ -100,11 +95,7 @@ __device__ __forceinline__ DualVals mri_dual_values(int W, int H, const ImgPtrs&
     a = pxo + sigma * (ux - c);
     b = pyo + sigma * (uy - c);
   }
-  DualVals o;
   const float sp = dual_proj_scale(sqrtf(abs2(a) + abs2(b)), alpha1);
-  o.px = a * sp;
-  o.py = b * sp;
-  o.qxx = o.qyy = o.qxy = c2(0.f, 0.f);
   if constexpr (TGV) {
     const float2 gxx = vxx - vx;
     const float2 gxy = 0.5f * (vxy - vx + vyx - vy);
@@ -113,29 +104,12 @@ __device__ __forceinline__ DualVals mri_dual_values(int W, int H, const ImgPtrs&
     const float2 qb = static_cast<const float2*>(in.qyy)[idx] + sigma * gyy;
     const float2 qc = static_cast<const float2*>(in.qxy)[idx] + sigma * gxy;
     const float sq = dual_proj_scale(sqrtf(abs2(qa) + abs2(qb) + 2.0f * abs2(qc)), alpha0);
-    o.qxx = qa * sq;
-    o.qyy = qb * sq;
-    o.qxy = qc * sq;
+    static_cast<float2*>(out.qxx)[idx] = qa * sq;
+    static_cast<float2*>(out.qyy)[idx] = qb * sq;
+    static_cast<float2*>(out.qxy)[idx] = qc * sq;
   }
-  return o;
-}
-
-template <bool TGV>
-__device__ __forceinline__ void store_dual(const ImgPtrs& out, size_t idx, const DualVals& d) {
-  static_cast<float2*>(out.px)[idx] = d.px;
-  static_cast<float2*>(out.py)[idx] = d.py;
-  if constexpr (TGV) {
-    static_cast<float2*>(out.qxx)[idx] = d.qxx;
-    static_cast<float2*>(out.qyy)[idx] = d.qyy;
-    static_cast<float2*>(out.qxy)[idx] = d.qxy;
-  }
-}
-
-// The dual update at pixel (x, y): u-bar, v-bar, p, q from `in`; p, q to `out`.
-template <bool TGV>
-__device__ __forceinline__ void mri_dual_pixel(int W, int H, const ImgPtrs& in, const ImgPtrs& out, float sigma,
-                                               float alpha0, float alpha1, int x, int y) {
-  store_dual<TGV>(out, (size_t)y * W + x, mri_dual_values<TGV>(W, H, in, sigma, alpha0, alpha1, x, y));
+  static_cast<float2*>(out.px)[idx] = a * sp;
+  static_cast<float2*>(out.py)[idx] = b * sp;
 }
 
 // The whole dual update spread over `nd` blocks of another kernel's grid (block `db` of them): pixels
