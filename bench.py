@@ -1056,6 +1056,25 @@ def run_ncu_case(args):
         print(json.dumps({"ncu_case": "radial_tgv2_12c_256x256_64spokes_x512", "iterations": args.ncu_iters}),
               flush=True)
         return
+    if args.ncu_workload == "denoising":
+        from primaldualtoolbox import synthetic
+
+        f = torch.from_numpy(synthetic.tv_phantom(512, 512, seed=0)[0]).cuda()
+        d = pdt.denoising
+        opts = [(d.TvOptimizer_2f(), f), (d.TgvOptimizer_2f(), f), (d.TgvOptimizer_2c(), torch.tile(f, (4, 4)).to(torch.complex64))]
+        for opt, img in opts:
+            prm = opt.getParameters()
+            prm.max_iter, prm.Lambda = args.ncu_iters - 1, 10.0
+            opt.setNoisyData(img, stream=stream)
+            opt.solve(stream=stream)
+        torch.cuda.synchronize()
+        torch.cuda.profiler.start()
+        for opt, _ in opts:
+            opt.solve(stream=stream)
+        torch.cuda.synchronize()
+        torch.cuda.profiler.stop()
+        print(json.dumps({"ncu_case": "denoising", "iterations": args.ncu_iters}), flush=True)
+        return
     case = _problem(seed=0)
     dev = {k: torch.from_numpy(np.ascontiguousarray(case[k])).cuda() for k in ("rawdata", "sens", "mask")}
     op = pdt.mri.MriCartesianRemoveROOSOperator()
@@ -1133,9 +1152,10 @@ def main():
     ap.add_argument("--radial-iters", type=int, default=200, help="radial leg: iterations per slice")
     ap.add_argument("--batch-cases", type=int, default=64, help="batched leg: independent problems (0 skips)")
     ap.add_argument("--batch-iters", type=int, default=200, help="batched leg: iterations per problem and step")
-    ap.add_argument("--ncu-workload", default="cartesian", choices=["cartesian", "radial", "cnn", "batched"],
+    ap.add_argument("--ncu-workload", default="cartesian", choices=["cartesian", "radial", "cnn", "batched", "denoising"],
                     help="profiling mode: the config-2 Cartesian problem, the config-5 radial slice, one "
-                         "training step of the warm-start network or the config-3 batch (--batch-cases)")
+                         "training step of the warm-start network, the config-3 batch (--batch-cases) or TV and TGV "
+                         "denoising of the 512 x 512 image and TGV of a 2048 x 2048 complex one")
     ap.add_argument("--ncu-iters", type=int, default=0,
                     help="profiling mode: one solve of this many iterations between cudaProfilerStart/Stop")
     args = ap.parse_args()
