@@ -34,8 +34,8 @@ struct RowsArgs {
 // through shared memory; rows of Y hold Q + 1 values so that both access directions are free of bank
 // conflicts. A row shift commutes with G, so the shifts of the operator's transforms drop out and slot x holds
 // image column x. The coil maps (used twice) arrive by asynchronous copies, the first pass's and the tables
-// before the programmatic wait and each further pass's during the one before it. Bound by the FMA pipe and
-// issue slots (15 coils, 320 x 368: 9.1 M warp instructions, 6.1 M of them on the FMA pipe) and by waves:
+// before the programmatic wait and each further pass's during the one before it. Bound by issue slots
+// and barriers (15 coils, 320 x 368: 7.1 M warp instructions, 4.0 M of them on the FMA pipe) and by waves:
 // 128 threads and five coils a block; with 96 or 64 threads and four or two coils 28.5 us an iteration.
 template <int P, int Q, int MINB>
 __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs a) {
@@ -153,8 +153,9 @@ __global__ void __launch_bounds__(kGramThreads, MINB) gram_rows_kernel(RowsArgs 
 // row kernel starts, and nothing the row kernel reads is written here, so the divergences, the v update and
 // the next q run before the programmatic wait (L2 loads: this SM may hold older lines). Bound by the latency
 // of its load phases: four blocks an SM (48 registers, some spilled) make one wave of the 480 blocks of a
-// 320 x 368 image and 17.6 us an iteration with the row kernel; three blocks 21.2, two 19.7 (before the product's
-// rounding error and the pair's remainder, which add 0.5).
+// 320 x 368 image and 17.6 us an iteration with the row kernel, solves one after the other; three blocks 21.2, two 19.7
+// (in a form with U for D). D, its compensation and w are loaded together with the sums: before the wait they took
+// registers (18.7 us an iteration against 17.9, set-up included).
 // ------------------------------------------------------------------------------------------------
 constexpr int GX = 32, GY = 8, GT = 320;  // (GX + 1) (GY + 1) = 297 primal pixels, one a thread
 
