@@ -1,7 +1,7 @@
 // pdt_cart_pair.cuh -- K^H (K u - f) of a line-sampled Cartesian operator in pairs of FP32 values (about 48 bits), once
 // per solve with the row operator (pdt_gram.h).
 //
-// The solve adds c times this image to K^H K U in every iteration, so an error of it acts in every iteration, also in
+// The solve adds c times this image to K^H K D in every iteration, so an error of it acts in every iteration, also in
 // the directions that the mask does not see, where nothing but the regularisation pulls it back. FP32 transforms are
 // 1.3e-7 off; with them a TGV-MRI solve (8 coils, 96 x 92, reduction 0.01) of 255 iterations ended 5.5e-7 off the
 // solution in 64 bits, where the k-space dual ends 2.1e-7 off. Pairs rather than FP64, whose units have a sixtieth of the
